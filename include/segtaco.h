@@ -21,7 +21,9 @@
  *
  * Scratch: entry points that need scratch memory take (workspace, bytes);
  * *_workspace_size() says how much.  workspace == NULL makes the library
- * allocate it stream-ordered (cudaMallocAsync/cudaFreeAsync) for that call.
+ * allocate it stream-ordered (cudaMallocAsync/cudaFreeAsync) for that call, from
+ * a pool of its own that keeps at most 64 MB per device between calls
+ * (segtaco_taco_release() gives it back).
  */
 #ifndef SEGTACO_H
 #define SEGTACO_H

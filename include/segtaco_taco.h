@@ -54,7 +54,8 @@ int segtaco_taco_call(const char *name, struct taco_tensor_t *out, struct taco_t
 float segtaco_taco_timer_ms(void);
 /* Device copies of the operands are kept per operand role and grown on
  * demand across calls (segTACO allocates and frees them per call); this frees
- * them. */
+ * them, and gives back the scratch that calls without a workspace keep (at
+ * most 64 MB per device). */
 void segtaco_taco_release(void);
 /* Number of names segtaco_taco_call accepts, and the i-th of them. */
 int segtaco_taco_num_names(void);

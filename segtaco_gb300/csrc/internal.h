@@ -42,6 +42,9 @@ class Scratch {
   size_t used_ = 0, total_ = 0;
 };
 
+// Gives the scratch kept between calls back to the driver.
+void trim_scratch_pools();
+
 inline size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
 // ---- launchers (partition.cu) ----

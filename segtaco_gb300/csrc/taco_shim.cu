@@ -599,6 +599,7 @@ void segtaco_taco_release(void) {
     if (slot.ptr) cudaFree(slot.ptr);
     slot = PoolSlot();
   }
+  segtaco::trim_scratch_pools();
 }
 int segtaco_taco_num_names(void) { return kNumEntries; }
 const char *segtaco_taco_name(int i) { return (i >= 0 && i < kNumEntries) ? kEntries[i].name : nullptr; }

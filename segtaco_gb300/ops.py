@@ -15,14 +15,23 @@ import torch
 from . import native as N
 
 
+# A small product's kernels take less time than its call from Python did (16,384
+# rows, N = 32: 9.4 us on the device, 12 us per call), so the calls below pass
+# plain integers, which ctypes converts by itself, and read the current stream's
+# handle without making a Stream object.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _ptr(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _stream(stream):
-    if stream is None:
-        stream = torch.cuda.current_stream()
-    return C.c_void_p(stream.cuda_stream)
+    if stream is not None:
+        return stream.cuda_stream
+    if _raw_stream is not None:
+        return _raw_stream(torch.cuda.current_device())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def _dense_dtype(t: torch.Tensor) -> int:
@@ -44,7 +53,7 @@ class DeviceCSR:
 
     @property
     def nnz(self) -> int:
-        return int(self.col.shape[0])
+        return self.col.size(0)
 
     @classmethod
     def from_host(cls, csr, device="cuda", with_values=True):
@@ -72,14 +81,14 @@ def spmm(A: DeviceCSR, B: torch.Tensor, C_out: torch.Tensor | None = None,
          config: N.Config | None = None, workspace: torch.Tensor | None = None,
          stream=None) -> torch.Tensor:
     """C = A @ B (B float32 or bfloat16, K x N row-major; C float32 M x N)."""
-    if B.dim() != 2 or B.shape[0] != A.K:
+    if B.dim() != 2 or B.size(0) != A.K:
         raise N.SegtacoError(N.EINVAL, "B must be K x N with K = %d" % A.K)
-    n = int(B.shape[1])
+    n = B.size(1)
     if C_out is None:
         C_out = torch.empty((A.M, n), dtype=torch.float32, device=B.device)
     ws_ptr, ws_bytes = None, 0
     if workspace is not None:
-        ws_ptr, ws_bytes = _ptr(workspace), workspace.numel() * workspace.element_size()
+        ws_ptr, ws_bytes = workspace.data_ptr(), workspace.nbytes
     N.check(N.lib().segtaco_spmm(A.M, A.K, A.nnz, _ptr(A.row_ptr), _ptr(A.col), _ptr(A.val),
                                  _ptr(B), _dense_dtype(B), B.stride(0), _ptr(C_out),
                                  C_out.stride(0), n, C.byref(config) if config else None,
