@@ -116,6 +116,53 @@ void *Scratch::take(size_t bytes) {
 // ---------------------------------------------------------------------------
 static bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
+// Merge-path chunks up to this many items take the split walk (a warp stages
+// its chunk in shared memory).
+constexpr long long kSplitMaxItems = 512;
+
+// The lane shape of the split walk (spmm_split.cuh) for N columns: E elements
+// per chunk (the widest load of at most 16 bytes that N, ldb and the pointers
+// allow: `fits`), C chunks per lane on G lanes.  False where no shape serves the
+// request: explicit narrow lanes, and fp32's 32-byte lanes, whose row walk is the
+// faster one for skewed rows over a B beyond L2 (1M x 1M power law, N = 128:
+// 1.10 ms against 1.18).
+template <typename F>
+static bool split_shape(const segtaco_config &c, int N, int K, int esz, F fits, SpmmPlan *plan) {
+  const int wide = 16 / esz;  // elements of a 16-byte chunk
+  if (c.vec > 0 && (c.vec < wide || (esz == 4 && c.vec > wide))) return false;
+  int E = wide;
+  while (E > 1 && !fits(E)) E >>= 1;
+  // Columns per slab: all of them up to 128, so that A is walked once and a slot's
+  // gather brings whole 128-byte lines.  Measured on GB300, lognormal rows (mean
+  // 12), fp32, slabs of 32 / 64 / 128 columns: 100,000 rows, N = 128, 71.6 / 56.9
+  // / 46.2 us; N = 127 109.9 / 85.3 / 69.7.  fp32 in 16-byte chunks over a B beyond
+  // L2: 64 (400,000 rows, N = 128: 258 / 253 / 280 us).
+  int cap = 128;
+  if (esz == 4 && E == wide && (double)K * N * esz > 96e6) cap = 64;
+  if (c.col_tile > 0 && c.col_tile < cap) cap = c.col_tile;
+  const int slabs = (N + cap - 1) / cap;
+  const int n = ((N + slabs - 1) / slabs + E - 1) / E;  // chunks of a slab
+  int C = 1, G;
+  if (E >= 4) {
+    G = 1;
+    while (G < 32 && 2 * G * E <= cap && G < n) G <<= 1;
+  } else if (n <= 8) {
+    G = 1;
+    while (G < n) G <<= 1;
+  } else {
+    // Several chunks per lane.  More lanes mean fewer 128-byte lines per load
+    // instruction and fewer slots: 77,777 rows, N = 37, 8 / 16 / 32 lanes 28.4 /
+    // 26.1 / 30.9 us; N = 17 20.4 / 23.1 / 28.3; N = 61 48.1 / 30.5 / 33.0.
+    G = n <= 24 ? 8 : n <= 64 && E == 1 ? 16 : 32;
+    C = (n + G - 1) / G;
+  }
+  plan->split_elems = E;
+  plan->V = E * C;
+  plan->G = G;
+  plan->W = G * E * C;
+  plan->slabs = (N + plan->W - 1) / plan->W;
+  return true;
+}
 
 int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, long long ldc,
               const void *B, const float *C, const segtaco_config *cfg, SpmmPlan *plan,
@@ -271,6 +318,13 @@ int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, lo
       plan->py_entries = 4;  // the two parts' counts, 64-bit work queue
     }
   }
+  // Merge-path chunks take the split walk unless another walk or a chunk beyond
+  // its staging is asked for.
+  if (eb && !plan->use_tma && plan->walk != 3 && plan->items_per_unit <= kSplitMaxItems &&
+      !(c.flags & (SEGTACO_FLAG_ROW_WALK | SEGTACO_FLAG_FLAT_WALK)) && c.depth != 8 &&
+      ldb * esz < (1LL << 32) && ldc * 4 < (1LL << 32) &&
+      split_shape(c, N, K, esz, fits, plan))
+    plan->walk = 5;
   plan->window_halo = -1;
   plan->band_halo = -1;
   if ((c.flags & SEGTACO_FLAG_WINDOW) && schedule == SEGTACO_RB_PR && plan->long_row == 0 &&
@@ -377,6 +431,11 @@ int run_spmm_planned(const SpmmPlan &plan, int M, int K, long long nnz, const in
         SEGTACO_TRY(launch_merge_path(row_ptr, M, nnz, plan.items_per_unit, plan.nchunks, px, py,
                                       C, ldc, N, s));
       if (L.use_tma) return bf16 ? launch_spmm_tma_bf16(L, false, s) : launch_spmm_tma_f32(L, false, s);
+      if (plan.walk == 5) {
+        L.split_elems = plan.split_elems;
+        L.split_items = (int)plan.items_per_unit;
+        return bf16 ? launch_spmm_split_bf16(L, s) : launch_spmm_split_f32(L, s);
+      }
       return bf16 ? launch_spmm_bf16_chunks(L, s) : launch_spmm_f32_chunks(L, s);
     default:
       return set_error(SEGTACO_EINVAL, "unknown schedule %d", plan.schedule);
@@ -466,6 +525,14 @@ int segtaco_autotune_heuristic(int32_t M, int32_t K, int64_t nnz, int32_t N, int
   // (4.38 ms).
   if (!sequential && esz == 4 && bbytes > 48e6 && N % 8 == 0 && (skewed || nnz >= 4000000))
     cfg->vec = 8;
+  // eb_pr takes the split walk with the planner's lanes (spmm_split.cuh) instead,
+  // unless most nonzeros are in long rows (a longest row of 256 means and more)
+  // over a B beyond L2.  Measured on GB300, N = 128, fp32, 8 columns per lane /
+  // split walk: 1M power-law rows 1.10 / 1.18 ms, 400,000 349 / 365 us; 400,000
+  // lognormal rows (longest 64 means) 380 / 250 us; B in L2 (250,000 power-law rows,
+  // N = 64) 120 / 105.
+  const bool heavy = (double)max_row_len > 256.0 * mean && bbytes > 96e6;
+  const bool split = schedule == SEGTACO_EB_PR && !(heavy && N % (32 / esz) == 0);
   // A B that fits L2 whole (up to ~96 MB) under a large product: one slab of
   // up to 64 columns (8 per lane, G = 8), so A is read once.  Measured on
   // GB300, banded 262,144 rows (19.1M nonzeros), N = 64, rb_pr: 0.248 ms
@@ -473,6 +540,7 @@ int segtaco_autotune_heuristic(int32_t M, int32_t K, int64_t nnz, int32_t N, int
   if (!sequential && esz == 4 && bbytes > 48e6 && bbytes <= 96e6 && nnz >= 4000000 &&
       N % 8 == 0 && !skewed)
     cfg->col_tile = N < 64 ? N : 64;
+  if (split) cfg->col_tile = cfg->vec = 0;
   // bf16 likewise: 16 columns per lane (one 32-byte load) on 64-column slabs.
   // Measured on GB300: 1M x 1M power law, N = 128, eb_pr 0.996 -> 0.823 ms;
   // with B in L2 (banded, N = 64) 8 stays faster (0.224 vs 0.235 ms).
@@ -669,6 +737,7 @@ static segtaco_config spmv_config() {
   c.col_tile = 1;
   c.vec = 1;
   c.items_per_unit = 512;
+  c.flags = SEGTACO_FLAG_ROW_WALK;
   return c;
 }
 

@@ -163,8 +163,22 @@ void fill_problem(BatchProblem<BT> &bp, const segtaco_spmm_problem &p, const Spm
   bp.index = index;
 }
 
-// Resident CTAs per SM of each batch kernel variant, per device (queried once).
-int blocks_per_sm(int device, int dtype, int V, int G, bool rows, int *out) {
+// Resident CTAs per SM of each batch kernel variant, per device (queried once;
+// the split walk's per launch shape, its shared memory follows the chunk size and
+// the number of problems).
+int blocks_per_sm(int device, const BatchLayout::Group &g, int *out) {
+  if (g.elems > 0) {
+    BatchGroupLaunch q{};
+    q.V = g.V;
+    q.G = g.G;
+    q.elems = g.elems;
+    q.items = g.items;
+    q.nprobs = (int)g.members.size();
+    return g.dtype == SEGTACO_BF16 ? batch_split_blocks_per_sm_bf16(q, out)
+                                   : batch_split_blocks_per_sm_f32(q, out);
+  }
+  const int dtype = g.dtype, V = g.V, G = g.G;
+  const bool rows = g.rows;
   static std::mutex mu;
   static std::map<std::tuple<int, int, int, int, bool>, int> cache;
   const auto key = std::make_tuple(device, dtype, V, G, rows);
@@ -202,13 +216,14 @@ int sm_count(int device) {
 void batch_layout(const segtaco_spmm_problem *probs, const SpmmPlan *plans, int count,
                   BatchLayout *L) {
   *L = BatchLayout();
-  std::map<std::tuple<int, int, int, bool>, int> gidx;
+  std::map<std::tuple<int, int, int, bool, int>, int> gidx;
   for (int i = 0; i < count; ++i) {
     const auto &p = probs[i];
     if (p.M == 0 || p.N == 0) continue;
     const auto &pl = plans[i];
     const bool rows = pl.schedule == SEGTACO_RB_SR || pl.schedule == SEGTACO_RB_PR;
-    const auto key = std::make_tuple(p.b_dtype, pl.V, pl.G, rows);
+    const int elems = pl.walk == kWalkSplit ? pl.split_elems : 0;
+    const auto key = std::make_tuple(p.b_dtype, pl.V, pl.G, rows, elems);
     auto it = gidx.find(key);
     if (it == gidx.end()) {
       it = gidx.emplace(key, (int)L->groups.size()).first;
@@ -217,9 +232,13 @@ void batch_layout(const segtaco_spmm_problem *probs, const SpmmPlan *plans, int 
       g.V = pl.V;
       g.G = pl.G;
       g.rows = rows;
+      g.elems = elems;
       L->groups.push_back(g);
     }
     L->groups[it->second].members.push_back(i);
+    if (elems > 0)
+      L->groups[it->second].items =
+          std::max(L->groups[it->second].items, (int)pl.items_per_unit);
   }
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -304,7 +323,7 @@ int batch_image(const segtaco_spmm_problem *probs, const SpmmPlan *plans, int co
     memcpy(img + g.off_begin, begin.data(), begin.size() * sizeof(long long));
     // Persistent grid: every SM full, never more CTAs than the items need.
     int per_sm = 0;
-    SEGTACO_TRY(blocks_per_sm(device, g.dtype, g.V, g.G, g.rows, &per_sm));
+    SEGTACO_TRY(blocks_per_sm(device, g, &per_sm));
     const long long need = (item + kSpmmWarps - 1) / kSpmmWarps;
     long long grid = (long long)std::max(1, per_sm) * std::max(1, sms);
     if (grid > need) grid = std::max(1LL, need);
@@ -343,6 +362,8 @@ int batch_enqueue(const BatchLayout &L, char *dbase, cudaStream_t s, const Batch
     G.V = g.V;
     G.G = g.G;
     G.rows = g.rows;
+    G.elems = g.elems;
+    G.items = g.items;
     G.probs = dbase + g.off_probs;
     G.item_begin = reinterpret_cast<const long long *>(dbase + g.off_begin);
     G.nprobs = (int)g.members.size();
@@ -350,7 +371,11 @@ int batch_enqueue(const BatchLayout &L, char *dbase, cudaStream_t s, const Batch
     G.queue = reinterpret_cast<unsigned long long *>(dbase + L.off_queues) + gi;
     G.grid = g.grid;
     G.gate = gate ? *gate : BatchGate{nullptr, 0, nullptr};
-    SEGTACO_TRY(g.dtype == SEGTACO_BF16 ? launch_batch_bf16(G, gs) : launch_batch_f32(G, gs));
+    if (g.elems > 0)
+      SEGTACO_TRY(g.dtype == SEGTACO_BF16 ? launch_batch_split_bf16(G, gs)
+                                          : launch_batch_split_f32(G, gs));
+    else
+      SEGTACO_TRY(g.dtype == SEGTACO_BF16 ? launch_batch_bf16(G, gs) : launch_batch_f32(G, gs));
     if (gs != s) {
       SEGTACO_TRY(check_cuda(cudaEventRecord(fork->join[gi], gs), "cudaEventRecord"));
       joined[gi] = 1;
@@ -387,15 +412,34 @@ int plan_batch_problem(const segtaco_spmm_problem &p, const segtaco_config *cfg,
     // chunks and row blocks that make one small product fill it alone.
     if (c.schedule == SEGTACO_RB_SR || c.schedule == SEGTACO_RB_PR) c.rows_per_unit = 4;
   }
-  if ((c.schedule == SEGTACO_EB_SR || c.schedule == SEGTACO_EB_PR) &&
-      (!cfg || c.items_per_unit <= 0))
-    c.items_per_unit = 512;
+  const bool eb = c.schedule == SEGTACO_EB_SR || c.schedule == SEGTACO_EB_PR;
+  if (eb && (!cfg || c.items_per_unit <= 0)) c.items_per_unit = 512;
   c.depth = 0;
   c.flags &= ~(SEGTACO_FLAG_SMEM_RING | SEGTACO_FLAG_TMA_BULK | SEGTACO_FLAG_PARTITION_READY);
   // The persistent kernel walks every row of its items (no long-row CTAs).
   c.flags &= ~SEGTACO_FLAG_LONG_ROWS;
+  SEGTACO_TRY(plan_spmm(p.M, p.K, p.nnz, p.N, p.b_dtype, p.ldb, p.ldc, p.B, p.C, &c, plan));
+  // The persistent kernel hides the row walk's round trips behind other problems'
+  // items, so the split walk pays there where it saves passes over A or narrow
+  // loads: slabs of more than 64 columns, and operands without 16-byte lanes, over
+  // chunks of 128 items.  Measured on GB300, the pool's problems of one N, row walk
+  // (slabs of up to 64 columns) / split walk at 128 and 256 items: N = 16 152 / 213
+  // / 187 us, 32 105 / 120 / 112, 64 131 / 131 / 129, 128 117 / 86 / 105.
+  if (plan->walk == kWalkSplit && !cfg) {
+    const int esz = p.b_dtype == SEGTACO_BF16 ? 2 : 4;
+    if (plan->split_elems * esz == 16 && plan->W <= 64) {
+      if (c.col_tile <= 0) c.col_tile = std::min(p.N, 256 / esz);
+      segtaco_config rows = c;
+      rows.flags |= SEGTACO_FLAG_ROW_WALK;
+      SEGTACO_TRY(
+          plan_spmm(p.M, p.K, p.nnz, p.N, p.b_dtype, p.ldb, p.ldc, p.B, p.C, &rows, plan));
+    } else if (c.items_per_unit > 128) {
+      c.items_per_unit = 128;
+      SEGTACO_TRY(plan_spmm(p.M, p.K, p.nnz, p.N, p.b_dtype, p.ldb, p.ldc, p.B, p.C, &c, plan));
+    }
+  }
   *used = c;
-  return plan_spmm(p.M, p.K, p.nnz, p.N, p.b_dtype, p.ldb, p.ldc, p.B, p.C, &c, plan);
+  return SEGTACO_OK;
 }
 
 }  // namespace segtaco

@@ -17,6 +17,7 @@
 
 #include "internal.h"
 #include "spmm_kernels.cuh"
+#include "spmm_split.cuh"
 
 namespace segtaco {
 
@@ -111,6 +112,41 @@ __global__ void __launch_bounds__(kSpmmCta, spmm_min_ctas<V, G, false>())
   }
 }
 
+// The split walk's items (merge-path chunks): as above, with each warp's chunk
+// staged in dynamic shared memory after the problems' item_begin values, and the
+// next item drawn while the current one is walked (the draw is a round trip to L2).
+// `D`: the largest chunk of the group's problems.
+template <typename BT, int E, int C, int G>
+__global__ void __launch_bounds__(kSpmmCta, split_min_ctas<BT, E, C, G>())
+    spmm_batch_split_kernel(const BatchProblem<BT> *__restrict__ probs,
+                            const long long *__restrict__ item_begin, int nprobs,
+                            long long total_items, unsigned long long *__restrict__ queue,
+                            BatchGate gate, int D) {
+  extern __shared__ __align__(16) int split_sm[];
+  const bool staged = nprobs <= kBatchSmemProblems;
+  long long *s_begin = reinterpret_cast<long long *>(split_sm + kSpmmWarps * split_words<E * C>(D));
+  if (staged)
+    for (int i = threadIdx.x; i < nprobs; i += blockDim.x) s_begin[i] = item_begin[i];
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  unsigned long long next = 0;
+  if (lane == 0) next = atomicAdd(queue, 1ULL);
+  for (;;) {
+    const unsigned long long item = __shfl_sync(0xffffffffu, next, 0);
+    if (item >= (unsigned long long)total_items) break;  // whole warp leaves together
+    if (lane == 0) next = atomicAdd(queue, 1ULL);
+    const int p = find_problem(staged ? s_begin : item_begin, nprobs, (long long)item);
+    const BatchProblem<BT> &bp = probs[p];
+    if (gate.gate != nullptr && !batch_gate_wait(gate, bp.index, lane)) break;
+    const long long local = (long long)item - bp.item_begin;
+    const long long units = bp.a.units;
+    const int slab = (int)(local / units);
+    spmm_split_unit<BT, E, C, G>(bp.a, local - (long long)slab * units, slab, lane, D,
+                                 split_sm + threadIdx.x / 32 * split_words<E * C>(D));
+    __syncwarp();  // the staging is free for the next item
+  }
+}
+
 // One thread per chunk edge over every element-balanced problem of the batch.
 struct BatchPartition {
   const int *row_ptr;
@@ -130,6 +166,8 @@ struct BatchPartition {
 struct BatchGroupLaunch {
   int V, G;
   bool rows;
+  int elems;  // > 0: the split walk, `elems` elements per lane chunk
+  int items;  // split walk: merge-path items of the largest chunk
   const void *probs;  // BatchProblem<BT>[nprobs] in device memory
   const long long *item_begin;
   int nprobs;
@@ -144,6 +182,8 @@ struct BatchLayout {
   struct Group {
     int dtype, V, G;
     bool rows;
+    int elems = 0;  // > 0: the split walk
+    int items = 0;  // split walk: merge-path items of the largest chunk
     std::vector<int> members;  // problem indices
     long long total_items = 0;
     size_t off_probs = 0, off_begin = 0;
@@ -192,5 +232,10 @@ int launch_batch_f32(const BatchGroupLaunch &g, cudaStream_t s);
 int launch_batch_bf16(const BatchGroupLaunch &g, cudaStream_t s);
 int batch_blocks_per_sm_f32(int V, int G, bool rows, int *out);
 int batch_blocks_per_sm_bf16(int V, int G, bool rows, int *out);
+// The split walk's groups (batch_split_<dtype>.cu).
+int launch_batch_split_f32(const BatchGroupLaunch &g, cudaStream_t s);
+int launch_batch_split_bf16(const BatchGroupLaunch &g, cudaStream_t s);
+int batch_split_blocks_per_sm_f32(const BatchGroupLaunch &g, int *out);
+int batch_split_blocks_per_sm_bf16(const BatchGroupLaunch &g, int *out);
 
 }  // namespace segtaco

@@ -398,6 +398,7 @@ template <int G> __device__ __forceinline__ unsigned group_mask(int lane) {
 }
 
 __device__ __forceinline__ int imin(int a, int b) { return a < b ? a : b; }
+__device__ __forceinline__ int imax(int a, int b) { return a > b ? a : b; }
 
 // Merge-path split of diagonal d over {row ends} U {nonzeros}: x = number of
 // row ends taken; row end x sorts before nonzero y when row_ptr[x+1] <= y.

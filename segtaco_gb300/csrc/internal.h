@@ -80,6 +80,8 @@ struct SpmmLaunch {
   int walk;                    // kWalkRows / kWalkRowsDeep / kWalkFlat (spmm_kernels.cuh)
   int long_row = 0;            // rb: rows of >= long_row nonzeros go to spmm_long.cu
   int carveout = -1;           // >= 0: preferred shared-memory carveout (%) of the launch
+  int split_elems = 0;         // split walk: elements per lane chunk (V / split_elems chunks)
+  int split_items = 0;         // split walk: merge-path items per chunk
   bool no_fork = false;        // rb long rows: both kernels on the call's stream (no side
                                // stream or events are created)
   int window_halo = -1;        // >= 0: rb rows with B rows [i0 - halo, i1 + halo) of each
@@ -105,6 +107,9 @@ int launch_spmm_f32_rows(const SpmmLaunch &L, cudaStream_t s);
 int launch_spmm_f32_chunks(const SpmmLaunch &L, cudaStream_t s);
 int launch_spmm_bf16_rows(const SpmmLaunch &L, cudaStream_t s);
 int launch_spmm_bf16_chunks(const SpmmLaunch &L, cudaStream_t s);
+// The split walk of merge-path chunks (spmm_split.cuh).
+int launch_spmm_split_f32(const SpmmLaunch &L, cudaStream_t s);
+int launch_spmm_split_bf16(const SpmmLaunch &L, cudaStream_t s);
 // rb_pr's pieces in piece_parts passes (a persistent launch before the row
 // blocks).
 int launch_spmm_pieces_f32(const SpmmLaunch &L, cudaStream_t s);
@@ -133,7 +138,8 @@ struct SpmmPlan {
   bool use_tma;
   bool bulk_copies;
   bool deep;
-  int walk;                  // kWalkRows / kWalkRowsDeep / kWalkFlat
+  int walk;                  // kWalkRows / kWalkRowsDeep / kWalkFlat / ... / kWalkSplit
+  int split_elems = 0;       // split walk: elements per lane chunk
   int long_row;              // rb: long-row threshold (0: every row in the row-block kernel)
   bool no_fork = false;      // rb long rows: no side stream (segtaco_spmm_noalloc)
   int window_halo = -1;      // rb: >= 0 stages each row block's B window (spmm_window.cu)
@@ -202,13 +208,14 @@ int launch_sddmm(int M, long long nnz, const int *row_ptr, const int *col, const
 // kernel: the list pass and the fork would cost more than a long row there.
 constexpr long long kLongRowsMinNnz = 1000000;
 // Merge-path items per chunk of a product launched alone: 512 (a warp's
-// chunk), halved down to 32 while the grid would hold fewer than 4,096
-// chunks, so that small products still fill the 152 SMs.  Measured on GB300,
-// 16,384 x 16,384 with 16 nonzeros per row, N = 32 (partition + product):
-// eb_sr 0.0462 -> 0.0240 ms and eb_pr 0.0295 -> 0.0203 ms with 64 items.
+// chunk), halved down to 32 while the grid would hold fewer than 3,072
+// chunks, so that small products still fill the 152 SMs.  Measured on GB300
+// (partition + product, split walk): 77,777 lognormal rows (1.02M items), N = 32,
+// 128 / 256 / 512 items 21.5 / 19.6 / 23.7 us; 20,000 rows (263K), N = 16, 64 /
+// 128 / 256 items 10.0 / 11.2 / 12.6 us.
 inline long long default_chunk_items(long long M, long long nnz) {
   long long D = 512;
-  while (D > 32 && (M + nnz) / D < 4096) D >>= 1;
+  while (D > 32 && (M + nnz) / D < 3072) D >>= 1;
   return D;
 }
 // Default long-row threshold (items_per_unit = 0).  Measured on GB300 (1M x 1M
