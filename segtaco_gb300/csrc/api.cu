@@ -785,10 +785,12 @@ int segtaco_sddmm_autotune(int32_t M, int32_t K, int64_t nnz, int32_t D, int32_t
   if (banded && D == 64) cfg->kernel = SEGTACO_SDDMM_BAND;
   (void)x_dtype;
   // Blocks of 256 nonzeros per warp; smaller for small problems, so that the
-  // launch still holds two waves of warps (152 SMs x 32 warps).
-  const long long two_waves = 2LL * 152 * 32;
+  // launch still holds about a wave of warps (152 SMs x 32).  Measured on GB300,
+  // default kernel, blocks of 32 / 64 / 128 / 256: 1.2M nonzeros, D = 16 - / 17.1 /
+  // 14.5 / 13.3 us, D = 64 bf16 - / 25.2 / 22.9 / 21.6; 58,751, D = 64 4.9 / 6.3 / 9.6
+  // / 16.8.
   int blk = 256;
-  while (blk > 32 && (nnz + blk - 1) / blk < two_waves) blk >>= 1;
+  while (blk > 32 && nnz / blk < 4096) blk >>= 1;
   cfg->block_nnz = blk;
   cfg->lanes = 0;  // from D (sddmm_shape)
   (void)max_row_len;
@@ -823,6 +825,17 @@ int segtaco_sddmm_ex(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr,
     return launch_sddmm_band(M, K, nnz, row_ptr, col, vals, X, Y, x_dtype, ldx, ldy, D, out, s);
   if (c.kernel == SEGTACO_SDDMM_BAND) c.kernel = SEGTACO_SDDMM_AUTO;
   const long long nblk = (nnz + P - 1) / P;
+  if (c.kernel == SEGTACO_SDDMM_AUTO && c.lanes == 0 && sddmm_gather_applies(x_dtype, ldx, ldy)) {
+    // Dot products of 512 bytes and more in 32-byte lanes stay with the fixed-shape
+    // kernel, two loads per lane (banded, 100,000 rows, D = 128 fp32: 219 us against
+    // 232; lognormal rows 55.5 / 55.7), also without a pass for the block starts.
+    const SddmmShape sh = sddmm_shape(x_dtype, D, ldx, ldy, X, Y, 0);
+    if ((sh.family == 1 || sh.family == 2) && sh.KI == 2 && sh.G >= 8)
+      return launch_sddmm(M, nnz, row_ptr, col, vals, X, Y, x_dtype, ldx, ldy, D, out, nullptr,
+                          (int)P, nblk, s, false, 0, SEGTACO_SDDMM_FIXED);
+    return launch_sddmm_gather(M, nnz, row_ptr, col, vals, X, Y, x_dtype, ldx, ldy, D, out, (int)P,
+                               nblk, s);
+  }
   Scratch scratch(nullptr, 0, s);
   SEGTACO_TRY(scratch.reserve(align256((size_t)(nblk + 1) * sizeof(int))));
   int *starts = static_cast<int *>(scratch.take((nblk + 1) * sizeof(int)));

@@ -198,6 +198,12 @@ bool sddmm_band_applies(int x_dtype, int D, long long ldx, long long ldy, const 
 int launch_sddmm_band(int M, int K, long long nnz, const int *row_ptr, const int *col,
                       const float *val, const void *X, const void *Y, int x_dtype, long long ldx,
                       long long ldy, int D, float *out, cudaStream_t s);
+// The default kernel (any D and alignment, row pitches below 4 GB; no scratch).
+bool sddmm_gather_applies(int x_dtype, long long ldx, long long ldy);
+int launch_sddmm_gather(int M, long long nnz, const int *row_ptr, const int *col,
+                        const float *val, const void *X, const void *Y, int x_dtype,
+                        long long ldx, long long ldy, int D, float *out, int P, long long nblk,
+                        cudaStream_t s);
 int launch_sddmm(int M, long long nnz, const int *row_ptr, const int *col, const float *val,
                  const void *X, const void *Y, int x_dtype, long long ldx, long long ldy, int D,
                  float *out, int *starts, int P, long long nblk, cudaStream_t s,

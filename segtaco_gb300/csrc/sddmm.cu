@@ -118,6 +118,195 @@ __global__ void __launch_bounds__(kCta, 3) sddmm_kernel(int M, long long nnz,
   }
 }
 
+// Last row r with row_ptr[r] <= p (the row of nonzero p), found by the whole warp:
+// 32 probes a round.  The first rounds' probes are the same for every warp and
+// stay in L1.
+__device__ __forceinline__ int warp_row_of(const int *__restrict__ row_ptr, int M, long long p,
+                                           int lane) {
+  long long lo = 0, hi = M;  // row_ptr[lo] <= p < row_ptr[hi]
+  while (hi - lo > 1) {
+    const long long step = (hi - lo + 31) / 32;
+    const long long at = lo + (lane + 1) * step;
+    const bool past = at >= hi || (long long)__ldg(row_ptr + at) > p;
+    const int f = __ffs(__ballot_sync(0xffffffffu, past)) - 1;  // lane 31's probe is past hi
+    const long long nhi = lo + (f + 1) * step;
+    lo += f * step;
+    hi = nhi < hi ? nhi : hi;
+  }
+  return (int)lo;
+}
+
+// The default kernel.  G lanes hold one dot product, each lane C chunks of E
+// elements (32 bytes where D, ldx, ldy and the pointers allow it, else 16, else one
+// or two elements), so the lanes of a group read whole lines of Y[j]; a group takes
+// U consecutive nonzeros per step and issues the loads of all of them, and of X for
+// the rows of its first and last nonzero, before the first multiply-add.  X stays
+// in registers while the row does.  The U sums over G lanes are reduced together,
+// each exchange halving the values a lane still holds (U = 4, G = 8: 4 shuffles
+// instead of 12).  FULL: D = G*E*C, so no lane is idle and one pass covers D;
+// otherwise idle chunks load zeros and D beyond G*E*C goes in passes.
+//
+// What bounds it: the gathers of Y, and for bf16 the instructions (two conversions
+// per multiply-add).  The row of a warp's first nonzero is searched in the kernel,
+// so a call is one launch and needs no scratch.  Measured on GB300, call time, the
+// kernels below (block starts, then the fixed-shape or general kernel) -> here:
+// 300,000 power-law rows, D = 128 bf16 196 -> 185 us, D = 64 fp32 170 -> 164; 100,000
+// lognormal rows, fp32, D = 16 / 32 17.9 -> 13.3, 24 -> 18; 85 204 -> 60; 40 84 -> 30;
+// 243,068 rows, D = 70 bf16 522 -> 79; 5000 rows, D = 64 19 -> 5.
+// U: 4, or 2 for 32-byte lanes on 8 lanes and more, which keeps 64 registers without
+// spills (300,000 power-law rows, D = 128 bf16: 185 us with 2, 221 with 4).
+template <int BYTES, int G> __host__ __device__ constexpr int sddmm_steps() {
+  return G < 4 ? G : BYTES == 32 && G >= 8 ? 2 : 4;
+}
+
+template <typename XT, int E, int C, int G, bool FULL>
+__global__ void __launch_bounds__(kCta, 4) sddmm_gather_kernel(
+    int M, unsigned nnz, const int *__restrict__ row_ptr, const int *__restrict__ col,
+    const float *__restrict__ val, const XT *__restrict__ X, const XT *__restrict__ Y,
+    unsigned ldx, unsigned ldy, int D, float *__restrict__ out, unsigned nblk, unsigned blk) {
+  constexpr int P = 32 / G;
+  constexpr int U = sddmm_steps<E * (int)sizeof(XT), G>();
+  using Dv = Dense<XT, E>;
+  const unsigned ALL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int g = lane / G, gl = lane & (G - 1);
+  const unsigned w = blockIdx.x * (kCta / 32) + threadIdx.x / 32;
+  if (w >= nblk) return;  // whole warp leaves together
+  const uint64_t pol = l2_policy_evict_normal();
+  const unsigned pb = w * blk;
+  const unsigned pe = nnz - pb < blk ? nnz : pb + blk;
+  auto load_cols = [&](unsigned p) { return p + lane < pe ? ld_stream(col + (p + lane)) : 0; };
+  auto load_vals = [&](unsigned p) {
+    return val && p + lane < pe ? ld_stream(val + (p + lane)) : 1.0f;
+  };
+  int mc = load_cols(pb);
+  float mv = load_vals(pb);
+  int wb = warp_row_of(row_ptr, M, pb, lane);
+  // ends of rows wb .. wb+31
+  unsigned rw = wb + lane < M ? (unsigned)__ldg(row_ptr + wb + 1 + lane) : 0xffffffffu;
+  // ldx and ldy are in bytes
+  const char *Xg = reinterpret_cast<const char *>(X + gl * E);
+  const char *Yg = reinterpret_cast<const char *>(Y + gl * E);
+  typename Dv::raw_t xa[C];  // X of row xrow (in one pass only)
+  int xrow = -1;
+  for (unsigned p = pb; p < pe; p += 32) {
+    const int nb = pe - p < 32 ? (int)(pe - p) : 32;
+    const int mcn = load_cols(p + 32);
+    const float mvn = load_vals(p + 32);
+    for (;;) {
+      const int adv = __popc(__ballot_sync(ALL, rw <= p));
+      if (adv == 0) break;
+      wb += adv;
+      rw = wb + lane < M ? (unsigned)__ldg(row_ptr + wb + 1 + lane) : 0xffffffffu;
+    }
+    // Row of nonzero p + lane (positions past the block: the block's last row).
+    const unsigned q = p + (lane < nb ? lane : nb - 1);
+    int myrow;
+    if (__shfl_sync(ALL, rw, 31) > p + (nb - 1)) {  // the window holds the batch
+      int rr = 0;
+#pragma unroll
+      for (int st = 16; st > 0; st >>= 1)
+        if (__shfl_sync(ALL, rw, rr + st - 1) <= q) rr += st;
+      myrow = wb + rr;
+    } else {
+      int lo = wb, hi = M - 1;
+      while (lo < hi) {
+        const int mid = lo + (hi - lo + 1) / 2;
+        if ((unsigned)__ldg(row_ptr + mid) <= q)
+          lo = mid;
+        else
+          hi = mid - 1;
+      }
+      myrow = lo;
+    }
+#pragma unroll 1
+    for (int s0 = 0; s0 < nb; s0 += P * U) {
+      const int t0 = s0 + g * U;  // this group's nonzeros t0 .. t0+U-1 of the batch
+      float sum[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) sum[u] = 0.0f;
+      const int r0 = __shfl_sync(ALL, myrow, t0), r1 = __shfl_sync(ALL, myrow, t0 + U - 1);
+      const bool one_row = U == 1 || __all_sync(ALL, r0 == r1);
+      for (int k0 = 0; k0 < (FULL ? 1 : D); k0 += FULL ? 1 : G * E * C) {
+        const int left = FULL ? D : D - k0 - gl * E;
+        const int chunks = left <= 0 ? 0 : imin(C, (left + G * E - 1) / (G * E));
+        const size_t kb = FULL ? 0 : (size_t)(left > 0 ? k0 : 0) * sizeof(XT);
+        auto load = [&](const char *base, int r, unsigned ld, typename Dv::raw_t(&d)[C]) {
+          const XT *p_ = reinterpret_cast<const XT *>(base + (size_t)(unsigned)r * ld + kb);
+#pragma unroll
+          for (int c = 0; c < C; ++c)
+            d[c] = FULL ? Dv::load(p_ + c * (G * E), pol)
+                        : Dv::load_if(p_ + c * (G * E), pol, c < chunks);
+        };
+        typename Dv::raw_t y[U][C];
+#pragma unroll
+        for (int u = 0; u < U; ++u) load(Yg, __shfl_sync(ALL, mc, t0 + u), ldy, y[u]);
+        if (r0 != xrow || (!FULL && D > G * E * C)) load(Xg, r0, ldx, xa);
+        auto dot = [&](int u) {
+#pragma unroll
+          for (int c = 0; c < C; ++c)
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+              sum[u] = fmaf(Dv::get(xa[c], e), Dv::get(y[u][c], e), sum[u]);
+        };
+        if (one_row) {
+#pragma unroll
+          for (int u = 0; u < U; ++u) dot(u);
+        } else {
+          typename Dv::raw_t xb[C];
+          load(Xg, r1, ldx, xb);
+          int at = r0;
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int r = __shfl_sync(ALL, myrow, t0 + u);
+            if (r != at) {
+              at = r;
+              if (r == r1) {
+#pragma unroll
+                for (int c = 0; c < C; ++c) xa[c] = xb[c];
+              } else {
+                load(Xg, r, ldx, xa);
+              }
+            }
+            __syncwarp();
+            dot(u);
+          }
+        }
+      }
+      xrow = r1;
+      // Sums over the group's lanes; lane gl ends with that of nonzero t0 + first.
+      int first = 0;
+      bool owner = true;
+      {
+        int n = U;
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) {
+          const bool hi = (lane & o) != 0;
+          if (n > 1) {
+            n /= 2;
+#pragma unroll
+            for (int i = 0; i < U / 2; ++i) {
+              if (i < n) {
+                const float keep = hi ? sum[i + n] : sum[i];
+                const float send = hi ? sum[i] : sum[i + n];
+                sum[i] = keep + __shfl_xor_sync(ALL, send, o);
+              }
+            }
+            if (hi) first += n;
+          } else {
+            sum[0] += __shfl_xor_sync(ALL, sum[0], o);
+            if (hi) owner = false;
+          }
+        }
+      }
+      const float v = __shfl_sync(ALL, mv, t0 + first);
+      if (owner && t0 + first < nb) out[p + (t0 + first)] = v * sum[0];
+    }
+    mc = mcn;
+    mv = mvn;
+  }
+}
+
 // Sixteen-byte vectors and D = G*V*KI: G lanes per dot product, each lane
 // KI vector loads of X[i] and of Y[j] (KI = 4 whenever D allows), so one step
 // covers P = 32/G nonzeros and its reduction takes only log2(G) shuffles.  The
@@ -139,7 +328,9 @@ __device__ __forceinline__ void sddmm_fixed_block(
   const uint64_t pol = l2_policy_evict_normal();
   const long long pb = w * blk;
   const long long pe = pb + blk < nnz ? pb + blk : nnz;
-  int wb = __ldg(starts + w);  // row of nonzero pb
+  int mcn = pb + lane < pe ? ld_stream(col + pb + lane) : 0;
+  float mvn = pb + lane < pe && val ? ld_stream(val + pb + lane) : 1.0f;
+  int wb = starts ? __ldg(starts + w) : warp_row_of(row_ptr, M, pb, lane);  // row of nonzero pb
   int rw = (wb + lane < M) ? __ldg(row_ptr + wb + 1 + lane) : INT_MAX;
   // The group's slice of X[xrow] stays in registers while its nonzeros stay in
   // that row (consecutive nonzeros of a row go to the same group's steps).
@@ -147,8 +338,10 @@ __device__ __forceinline__ void sddmm_fixed_block(
   int xrow = -1;
   for (long long p = pb; p < pe; p += 32) {
     const int nb = (int)(pe - p < 32 ? pe - p : 32);
-    const int mc = lane < nb ? ld_stream(col + p + lane) : 0;
-    const float mv = lane < nb ? (val ? ld_stream(val + p + lane) : 1.0f) : 0.0f;
+    const int mc = mcn;  // columns and values of this batch; the next one's load meanwhile
+    const float mv = mvn;
+    mcn = p + 32 + lane < pe ? ld_stream(col + p + 32 + lane) : 0;
+    mvn = p + 32 + lane < pe && val ? ld_stream(val + p + 32 + lane) : 1.0f;
     for (;;) {
       const int adv = __popc(__ballot_sync(FULL, (long long)rw <= p));
       if (adv == 0) break;
@@ -357,12 +550,92 @@ int launch_fixed_multi(const SddmmShape &sh, int x_dtype, dim3 grid, const Sddmm
                                                  starts, nblk, P);                            \
     break;
 
+// Lane shapes (E, C, G) of the default kernel: 32- and 16-byte chunks (bf16: and
+// 8-byte ones), one per lane, and one to four 1- or 2-element chunks.
+#define SEGTACO_SDDMM_NARROW(X_, XT, E) \
+  X_(XT, E, 1, 1) X_(XT, E, 1, 2) X_(XT, E, 1, 4) X_(XT, E, 1, 8) X_(XT, E, 2, 8) X_(XT, E, 3, 8) \
+  X_(XT, E, 4, 8) X_(XT, E, 5, 8) X_(XT, E, 3, 16) X_(XT, E, 4, 16) X_(XT, E, 2, 32) X_(XT, E, 3, 32) \
+  X_(XT, E, 4, 32)
+#define SEGTACO_SDDMM_WIDE(X_, XT, E) \
+  X_(XT, E, 1, 1) X_(XT, E, 1, 2) X_(XT, E, 1, 4) X_(XT, E, 1, 8) X_(XT, E, 1, 16) X_(XT, E, 1, 32)
+#define SEGTACO_SDDMM_KEY(E, C, G) ((E)*10000 + (C)*100 + (G))
+#define SEGTACO_SDDMM_RUN(XT, E, C, G, F)                                                  \
+  sddmm_gather_kernel<XT, E, C, G, F><<<grid, kCta, 0, s>>>(                               \
+      M, (unsigned)nnz, row_ptr, col, val, static_cast<const XT *>(X),                     \
+      static_cast<const XT *>(Y), (unsigned)(ldx * sizeof(XT)), (unsigned)(ldy * sizeof(XT)), D, \
+      out, (unsigned)nblk, (unsigned)P)
+#define SEGTACO_SDDMM_NARROW_CASE(XT, E, C, G)  \
+  case SEGTACO_SDDMM_KEY(E, C, G):              \
+    SEGTACO_SDDMM_RUN(XT, E, C, G, false);      \
+    break;
+#define SEGTACO_SDDMM_WIDE_CASE(XT, E, C, G)    \
+  case SEGTACO_SDDMM_KEY(E, C, G):              \
+    if (D == (E) * (C) * (G))                   \
+      SEGTACO_SDDMM_RUN(XT, E, C, G, true);     \
+    else                                        \
+      SEGTACO_SDDMM_RUN(XT, E, C, G, false);    \
+    break;
+
+bool sddmm_gather_applies(int x_dtype, long long ldx, long long ldy) {
+  const int esz = x_dtype == SEGTACO_BF16 ? 2 : 4;
+  return ldx * esz < (1LL << 32) && ldy * esz < (1LL << 32);
+}
+
+int launch_sddmm_gather(int M, long long nnz, const int *row_ptr, const int *col,
+                        const float *val, const void *X, const void *Y, int x_dtype,
+                        long long ldx, long long ldy, int D, float *out, int P, long long nblk,
+                        cudaStream_t s) {
+  const dim3 grid((unsigned)((nblk + (kCta / 32) - 1) / (kCta / 32)));
+  const int esz = x_dtype == SEGTACO_BF16 ? 2 : 4;
+  const uintptr_t al = (uintptr_t)X | (uintptr_t)Y;
+  int E = 32 / esz;
+  while (E > 1 && (D % E != 0 || ldx % E != 0 || ldy % E != 0 || (al % (E * esz)) != 0)) E >>= 1;
+  // As many lanes as D needs chunks of 16 and 32 bytes; fewer lanes with up to five
+  // chunks of 1 and 2 elements each (more nonzeros per step), until a load
+  // instruction would touch too many lines.  Measured on GB300, 100,000 lognormal
+  // rows (1.2M nonzeros), fp32, 8 / 16 / 32 lanes: D = 17 24.0 / 32.3 / 47.8 us, 37
+  // 32.1 / 35.4 / 51.4, 61 57.0 / 39.4 / 51.8, 127 - / 85.3 / 70.0.
+  const int n = (D + E - 1) / E;
+  int C = 1, G = 1;
+  if (E == 4 && esz == 2 && n > 16 && n <= 32) {
+    G = 16, C = 2;  // bf16 in 8-byte chunks: D = 100 44 us against 58 with 32 lanes
+  } else if (E >= 4 || n <= 8) {
+    while (G < 32 && G < n) G <<= 1;
+  } else {
+    G = n <= 40 ? 8 : n <= 64 && E == 1 ? 16 : 32;
+    C = (n + G - 1) / G;
+    if (C > 4 && G == 32) C = 4;
+  }
+  if (x_dtype == SEGTACO_BF16) {
+    switch (SEGTACO_SDDMM_KEY(E, C, G)) {
+      SEGTACO_SDDMM_WIDE(SEGTACO_SDDMM_WIDE_CASE, uint16_t, 16)
+      SEGTACO_SDDMM_WIDE(SEGTACO_SDDMM_WIDE_CASE, uint16_t, 8)
+      SEGTACO_SDDMM_WIDE(SEGTACO_SDDMM_NARROW_CASE, uint16_t, 4)
+      SEGTACO_SDDMM_NARROW_CASE(uint16_t, 4, 2, 16)
+      SEGTACO_SDDMM_NARROW(SEGTACO_SDDMM_NARROW_CASE, uint16_t, 2)
+      SEGTACO_SDDMM_NARROW(SEGTACO_SDDMM_NARROW_CASE, uint16_t, 1)
+      default:
+        return set_error(SEGTACO_EUNSUPPORTED, "sddmm: no bf16 shape E=%d C=%d G=%d", E, C, G);
+    }
+  } else {
+    switch (SEGTACO_SDDMM_KEY(E, C, G)) {
+      SEGTACO_SDDMM_WIDE(SEGTACO_SDDMM_WIDE_CASE, float, 8)
+      SEGTACO_SDDMM_WIDE(SEGTACO_SDDMM_WIDE_CASE, float, 4)
+      SEGTACO_SDDMM_NARROW(SEGTACO_SDDMM_NARROW_CASE, float, 2)
+      SEGTACO_SDDMM_NARROW(SEGTACO_SDDMM_NARROW_CASE, float, 1)
+      default:
+        return set_error(SEGTACO_EUNSUPPORTED, "sddmm: no f32 shape E=%d C=%d G=%d", E, C, G);
+    }
+  }
+  return check_launch("sddmm_gather_kernel");
+}
+
 int launch_sddmm(int M, long long nnz, const int *row_ptr, const int *col, const float *val,
                  const void *X, const void *Y, int x_dtype, long long ldx, long long ldy, int D,
                  float *out, int *starts, int P, long long nblk, cudaStream_t s,
                  bool starts_ready, int lanes, int kernel) {
   if (nnz == 0) return SEGTACO_OK;
-  if (!starts_ready)
+  if (!starts_ready && starts)
     SEGTACO_TRY(launch_block_starts_canonical(row_ptr, M, P, nblk, starts, s));
   const dim3 grid((unsigned)((nblk + (kCta / 32) - 1) / (kCta / 32)));
   // The fixed-shape kernel where D and the operands allow it (unless the
