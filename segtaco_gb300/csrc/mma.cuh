@@ -1,0 +1,56 @@
+// mma.cuh -- warp-level tensor-core steps of the band kernels (bf16 operands, fp32
+// accumulation) and the exact split of fp32 values into bf16 parts.
+#pragma once
+
+#include <stdint.h>
+
+namespace segtaco {
+
+// x = hi + mid + lo for two values, each part a bf16 pair (truncation: exact).
+__device__ __forceinline__ void split3(float x, float y, uint32_t &hi, uint32_t &mid,
+                                       uint32_t &lo) {
+  const uint32_t xb = __float_as_uint(x), yb = __float_as_uint(y);
+  hi = __byte_perm(xb, yb, 0x7632);
+  const float xr = x - __uint_as_float(xb & 0xffff0000u);
+  const float yr = y - __uint_as_float(yb & 0xffff0000u);
+  const uint32_t xm = __float_as_uint(xr), ym = __float_as_uint(yr);
+  mid = __byte_perm(xm, ym, 0x7632);
+  lo = __byte_perm(__float_as_uint(xr - __uint_as_float(xm & 0xffff0000u)),
+                   __float_as_uint(yr - __uint_as_float(ym & 0xffff0000u)), 0x7632);
+}
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
+                                         uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// d = a x b (from zero).
+__device__ __forceinline__ void mma_bf16_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
+                                              uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
+// The larger magnitude (its sign is no use), NaN if either is NaN.
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t max_nan_bf16(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+
+}  // namespace segtaco

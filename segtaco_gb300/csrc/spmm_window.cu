@@ -25,6 +25,7 @@
 #include <atomic>
 #include <mutex>
 
+#include "mma.cuh"
 #include "spmm_launch.cuh"
 
 namespace segtaco {
@@ -102,7 +103,8 @@ __global__ void __launch_bounds__(kSpmmCta, window_min_ctas<BT, V, G>())
 }
 
 // ---------------------------------------------------------------------------
-// Banded row blocks for rb_pr (SEGTACO_FLAG_WINDOW with a parallel reduction).
+// Banded row blocks for rb_pr (SEGTACO_FLAG_WINDOW with a parallel reduction), fp32
+// B; bf16 B: spmm_band_mma_kernel below.
 //
 // On a banded matrix the plain row blocks deliver each nonzero's 64-column B
 // slice to registers (256 bytes for 64 multiply-adds), and that load/store
@@ -133,23 +135,8 @@ constexpr int kBandCols = 64;
 constexpr int kBandList = 16;
 constexpr int kBandPitch = 36;
 
-// Four consecutive B values as floats: from shared memory, or from global
-// memory through the read-only path.
-template <typename BT> __device__ __forceinline__ float4 band_b4(const BT *p) {
-  if constexpr (sizeof(BT) == 4) {
-    return *reinterpret_cast<const float4 *>(p);
-  } else {
-    const uint2 x = *reinterpret_cast<const uint2 *>(p);
-    return make_float4(bf16lo(x.x), bf16hi(x.x), bf16lo(x.y), bf16hi(x.y));
-  }
-}
-template <typename BT> __device__ __forceinline__ float4 band_b4_global(const BT *p) {
-  if constexpr (sizeof(BT) == 4) {
-    return __ldg(reinterpret_cast<const float4 *>(p));
-  } else {
-    const uint2 x = __ldg(reinterpret_cast<const uint2 *>(p));
-    return make_float4(bf16lo(x.x), bf16hi(x.x), bf16lo(x.y), bf16hi(x.y));
-  }
+__device__ __forceinline__ float4 band_b4(const float *p) {
+  return __ldg(reinterpret_cast<const float4 *>(p));
 }
 __device__ __forceinline__ void band_fma4(float (&acc)[4], float x, const float4 &b) {
   acc[0] = fmaf(x, b.x, acc[0]);
@@ -162,9 +149,9 @@ __device__ __forceinline__ void band_fma4(float (&acc)[4], float x, const float4
 struct BandSmem {
   size_t at, rp, cnt, lcol, lval, bar, bytes;
 };
-template <typename BT> __host__ __device__ inline BandSmem band_smem(int win) {
+__host__ __device__ inline BandSmem band_smem(int win) {
   BandSmem m;
-  size_t o = ((size_t)win * kBandCols * sizeof(BT) + 127) & ~size_t(127);  // B window first
+  size_t o = ((size_t)win * kBandCols * sizeof(float) + 127) & ~size_t(127);  // B window first
   m.at = o;
   o += (size_t)win * kBandPitch * 4;
   m.rp = o;
@@ -180,14 +167,13 @@ template <typename BT> __host__ __device__ inline BandSmem band_smem(int win) {
   return m;
 }
 
-template <typename BT>
 __global__ void __launch_bounds__(kSpmmCta)
-    spmm_band_kernel(SpmmArgs<BT> a, const __grid_constant__ CUtensorMap tm, int halo,
+    spmm_band_kernel(SpmmArgs<float> a, const __grid_constant__ CUtensorMap tm, int halo,
                      int *status) {
   const int win = kBandRows + 2 * halo;
-  const BandSmem L = band_smem<BT>(win);
+  const BandSmem L = band_smem(win);
   extern __shared__ __align__(128) unsigned char smem[];
-  BT *bw = reinterpret_cast<BT *>(smem);  // [win][kBandCols]
+  float *bw = reinterpret_cast<float *>(smem);  // [win][kBandCols]
   float *at = reinterpret_cast<float *>(smem + L.at);  // [win][kBandPitch]
   int *rp = reinterpret_cast<int *>(smem + L.rp);
   int *cnt = reinterpret_cast<int *>(smem + L.cnt);
@@ -209,7 +195,7 @@ __global__ void __launch_bounds__(kSpmmCta)
   if (t < kBandRows) cnt[t] = 0;
   __syncthreads();
   if (t == 0) {
-    const uint32_t bytes = (uint32_t)((size_t)win * kBandCols * sizeof(BT));
+    const uint32_t bytes = (uint32_t)((size_t)win * kBandCols * sizeof(float));
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes)
                  : "memory");
     // x = the slab's first column (a multiple of 64 elements), y = the
@@ -275,14 +261,14 @@ __global__ void __launch_bounds__(kSpmmCta)
   for (int e = 0; e < 8; ++e) {
     // slots past the row's list gather B row 0 (in bounds) and are not used
     const int j = e < pre ? lcol[4 * rb * kBandList + e] : 0;
-    g0[e] = band_b4_global<BT>(a.B + (size_t)(unsigned)j * a.ldb + c0);
+    g0[e] = band_b4(a.B + (size_t)(unsigned)j * a.ldb + c0);
   }
   const float *acol = at + 4 * rb;
-  const BT *bcol = bw + 4 * cb;
+  const float *bcol = bw + 4 * cb;
 #pragma unroll 4
   for (int j = 0; j < win; ++j) {
     const float4 x = *reinterpret_cast<const float4 *>(acol + j * kBandPitch);
-    const float4 bv = band_b4<BT>(bcol + j * kBandCols);
+    const float4 bv = *reinterpret_cast<const float4 *>(bcol + j * kBandCols);
     band_fma4(acc[0], x.x, bv);
     band_fma4(acc[1], x.y, bv);
     band_fma4(acc[2], x.z, bv);
@@ -302,7 +288,7 @@ __global__ void __launch_bounds__(kSpmmCta)
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const int ee = e0 + e < n ? e0 + e : e0;
-          g[e] = band_b4_global<BT>(a.B + (size_t)(unsigned)lcol[r * kBandList + ee] * a.ldb + c0);
+          g[e] = band_b4(a.B + (size_t)(unsigned)lcol[r * kBandList + ee] * a.ldb + c0);
         }
 #pragma unroll
         for (int e = 0; e < 8; ++e)
@@ -314,7 +300,7 @@ __global__ void __launch_bounds__(kSpmmCta)
         const int j = __ldg(a.col + k);
         if ((unsigned)(j - jw0) >= (unsigned)win)
           band_fma4(acc[q], ld_val(a.val, k),
-                    band_b4_global<BT>(a.B + (size_t)(unsigned)j * a.ldb + c0));
+                    band_b4(a.B + (size_t)(unsigned)j * a.ldb + c0));
       }
     }
   }
@@ -324,6 +310,259 @@ __global__ void __launch_bounds__(kSpmmCta)
     if (i < M)
       __stcs(reinterpret_cast<float4 *>(a.C + (long long)i * a.ldc + c0),
              make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The band tile on the tensor cores, for a bf16 dense operand.
+//
+// The tile product At x B is a dense contraction (32 x win by win x 64 per CTA), and
+// its multiply-adds, two shared loads per 16 of them, were the kernel's time.  Here
+// it runs as mma.m16n8k16 with fp32 accumulation.  A's values are fp32: each is cut
+// exactly into three bf16 parts of 8 bits (x = hi + mid + lo, truncating), so three
+// products per step give the exact products x*b that the multiply-add form rounds
+// once; the parts of a step are summed from zero, lowest first, and added to the
+// running sum in fp32.  (tcgen05 needs 64 or 128 rows per tile: a 32-row block's
+// band fills 68 % of its 96-column window, a 128-row block's 34 % of 192.)
+//
+// Warp w: rows 16 (w & 1) .. +15, all 64 columns, every other half of the window
+// steps (w >> 1).  B's window comes by TMA with the 128-byte swizzle and is read
+// with ldmatrix.trans.  The two halves' sums go to shared memory (the tile's space),
+// and eight lanes per row then add its off-band nonzeros (16 bytes of B per lane) and
+// store whole lines of C.
+//
+// Splitting an infinity or NaN, or multiplying a zero part by one, would make NaN:
+// a CTA that meets one in its tile or window sums its rows nonzero by nonzero
+// instead.
+//
+// What bounds it now: instructions (58 % of issue slots with 24 warps per SM), most of
+// them in the scatter and the off-band rows; the tensor pipe is 14 % busy.  Measured
+// on GB300, banded-plus-random 262,144 rows (half band 32, 8 off-band nonzeros per
+// row), bf16 B, N = 64: 160 us with multiply-adds -> 114 (without the product 97,
+// without the off-band rows 97); error against FP64 1.5e-7 -> 9.3e-8.  20 nonzeros in
+// flight per thread instead of 10 117.5 -> 115.6 us; a warp per row instead of the flat
+// scatter 122; seven CTAs per SM 120; all three parts summed in the tensor cores'
+// accumulators 120 us and an error of 1.57e-7.
+constexpr int kBandAPad = 8;   // tile pitch win + 8: conflict-free 8-byte fragment loads
+constexpr int kBandCPad = 4;   // pitch of the summed rows: 68 floats
+
+struct BandMmaSmem {
+  size_t at, list, rp, cnt, bar, bytes;
+};
+__host__ __device__ inline int band_mma_win(int halo) { return (kBandRows + 2 * halo + 15) & ~15; }
+__host__ __device__ inline BandMmaSmem band_mma_smem(int win) {
+  BandMmaSmem m;
+  m.at = (size_t)win * 128;  // B window first: 64 bf16 per row
+  size_t o = m.at + (size_t)kBandRows * (win + kBandAPad) * 4;
+  const size_t sums = (size_t)2 * kBandRows * (kBandCols + kBandCPad) * 4;
+  if (o < sums) o = sums;
+  m.list = o;  // (column, value bits)
+  o += (size_t)kBandRows * kBandList * 8;
+  m.rp = o;
+  o += (kBandRows + 1) * 4;
+  m.cnt = o;
+  o += kBandRows * 4;
+  m.bar = (o + 7) & ~size_t(7);
+  m.bytes = m.bar + 8;
+  return m;
+}
+
+__global__ void __launch_bounds__(kSpmmCta, 6)
+    spmm_band_mma_kernel(SpmmArgs<uint16_t> a, const __grid_constant__ CUtensorMap tm, int halo,
+                         int *status) {
+  const int win = band_mma_win(halo);
+  const int pitch = win + kBandAPad;
+  const BandMmaSmem L = band_mma_smem(win);
+  extern __shared__ __align__(1024) unsigned char swz[];  // the 128-byte swizzle's period
+  float *at = reinterpret_cast<float *>(swz + L.at);  // [kBandRows][pitch]
+  float *sums = reinterpret_cast<float *>(swz);       // [2][kBandRows][68], after the product
+  int2 *list = reinterpret_cast<int2 *>(swz + L.list);
+  int *rp = reinterpret_cast<int *>(swz + L.rp);
+  int *cnt = reinterpret_cast<int *>(swz + L.cnt);
+  uint64_t *bar = reinterpret_cast<uint64_t *>(swz + L.bar);
+  const int t = threadIdx.x, lane = t & 31;
+  const int M = a.M;
+  const int i0 = blockIdx.x * kBandRows;
+  const int jw0 = (int)((long long)i0 * a.K / M) - halo;
+  const uint32_t b = sm_u32(bar);
+  if (t == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b),
+                 "r"((uint32_t)(win * 128))
+                 : "memory");
+    // x = the slab's first column (a multiple of 64 elements), y = the
+    // window's first row (negative at the top edge: zero-filled)
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3}], [%4];" ::"r"(sm_u32(swz)),
+        "l"(&tm), "r"((int)(blockIdx.y * kBandCols)), "r"(jw0), "r"(b)
+        : "memory");
+  }
+  // Scatter the block's nonzeros, SQ per thread per pass with every load in flight;
+  // the first pass loads before the tile is cleared.  An exchange puts a value in
+  // the tile; where it returns another entry of the same position, that one is added
+  // back (the native exchange is one instruction, an add of floats in shared memory a
+  // loop).
+  constexpr int SQ = 20;
+  const int k_beg = __ldg(a.row_ptr + i0), k_end = __ldg(a.row_ptr + min(i0 + kBandRows, M));
+  int cj[SQ];
+  float cv[SQ];
+  auto load = [&](int n0) {  // nonzeros k_beg + n0 + t + 128 q
+#pragma unroll
+    for (int q = 0; q < SQ; ++q) {
+      const bool has = n0 + t + q * kSpmmCta < k_end - k_beg;
+      cj[q] = has ? __ldg(a.col + (k_beg + n0 + t + q * kSpmmCta)) : 0;
+      cv[q] = has ? ld_val(a.val, k_beg + n0 + t + q * kSpmmCta) : 0.0f;
+    }
+  };
+  load(0);
+  for (int e = t; e < kBandRows * pitch / 4; e += kSpmmCta)
+    reinterpret_cast<float4 *>(at)[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (t <= kBandRows) rp[t] = __ldg(a.row_ptr + min(i0 + t, M));
+  if (t < kBandRows) cnt[t] = 0;
+  __syncthreads();
+  float amax = 0.0f;  // the tile's largest magnitude, or NaN
+  for (int n0 = 0; n0 < k_end - k_beg; n0 += SQ * kSpmmCta) {
+    if (n0 > 0) load(n0);
+    int r = 0;  // the last row whose start is <= the thread's first nonzero
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (r + step <= kBandRows - 1 && rp[r + step] - k_beg <= n0 + t) r += step;
+    int rend = rp[r + 1] - k_beg;
+#pragma unroll
+    for (int q = 0; q < SQ; ++q) {
+      const int n = n0 + t + q * kSpmmCta;
+      if (n < k_end - k_beg) {
+        while (n >= rend) rend = rp[++r + 1] - k_beg;  // n < rp[kBandRows] - k_beg
+        const unsigned d = (unsigned)(cj[q] - jw0);
+        if (d < (unsigned)win) {
+          float *cell = at + r * pitch + d;
+          const float old = atomicExch(cell, cv[q]);
+          if (old != 0.0f) atomicAdd(cell, old);
+          amax = max_nan(amax, cv[q]);
+        } else {
+          const int slot = atomicAdd(cnt + r, 1);
+          if (slot < kBandList) list[r * kBandList + slot] = make_int2(cj[q], __float_as_int(cv[q]));
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (!window_wait(b)) {
+    if (t == 0) atomicExch(status, SEGTACO_ETIMEOUT);
+    window_wait(b);  // the copy may still land: wait for it once more, bounded
+    return;
+  }
+  // ---- the tile product --------------------------------------------------
+  float acc[8][4];
+#pragma unroll
+  for (int n = 0; n < 8; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+  const int w = t >> 5;
+  const int steps = win / 16, half = (steps + 1) / 2;
+  const int s0 = w < 2 ? 0 : half, s1 = w < 2 ? half : steps;
+  // A fragment: rows 16 (w & 1) + lane / 4 (and + 8), columns 2 (lane % 4) (and + 8)
+  const float *arow = at + (16 * (w & 1) + (lane >> 2)) * pitch + 2 * (lane & 3);
+  // B fragments of two n-tiles: lanes 0-15 rows k .. k+15 of columns 8n, 16-31 of 8n + 8
+  const uint32_t brow = sm_u32(swz) + (uint32_t)(lane & 15) * 128;
+  uint32_t bmax = 0;  // the window's largest magnitudes (bf16 pairs), or NaN
+#pragma unroll 1
+  for (int s = s0; s < s1; ++s) {
+    uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // a0: row, a1: row + 8, a2, a3: columns + 8
+      const float2 v =
+          *reinterpret_cast<const float2 *>(arow + (q & 1) * 8 * pitch + 16 * s + (q >> 1) * 8);
+      amax = max_nan(max_nan(amax, v.x), v.y);
+      split3(v.x, v.y, hi[q], mid[q], lo[q]);
+    }
+    const uint32_t row = brow + (uint32_t)s * 16 * 128;
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) {
+      uint32_t bf[4];
+      ldmatrix_x4_trans(bf, row + ((((uint32_t)(2 * n2 + (lane >> 4))) ^ ((row >> 7) & 7)) << 4));
+#pragma unroll
+      for (int q = 0; q < 4; ++q) bmax = max_nan_bf16(bmax, bf[q]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float d[4];
+        mma_bf16_zero(d, lo, bf[2 * h], bf[2 * h + 1]);
+        mma_bf16(d, mid, bf[2 * h], bf[2 * h + 1]);
+        mma_bf16(d, hi, bf[2 * h], bf[2 * h + 1]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[2 * n2 + h][q] += d[q];
+      }
+    }
+  }
+  // An exponent of all ones: infinity or NaN.
+  const bool odd = !(fabsf(amax) <= 3.402823466e38f) || (bmax & 0x7f80u) == 0x7f80u ||
+                   (bmax & 0x7f800000u) == 0x7f800000u;
+  const bool direct = __syncthreads_or(odd) != 0;  // the tile and the window are free now
+  {
+    float *s = sums + (w >> 1) * kBandRows * (kBandCols + kBandCPad) +
+               (16 * (w & 1) + (lane >> 2)) * (kBandCols + kBandCPad) + 2 * (lane & 3);
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      *reinterpret_cast<float2 *>(s + 8 * n) = make_float2(acc[n][0], acc[n][1]);
+      *reinterpret_cast<float2 *>(s + 8 * (kBandCols + kBandCPad) + 8 * n) =
+          make_float2(acc[n][2], acc[n][3]);
+    }
+  }
+  __syncthreads();
+  // ---- off-band nonzeros and the store: eight lanes per row, 8 columns each ----
+  const int l = t & 7;
+  const int c0 = blockIdx.y * kBandCols + 8 * l;
+  if (c0 >= a.N) return;  // N is a multiple of 16
+  auto gather = [&](int j) {
+    return __ldg(reinterpret_cast<const uint4 *>(a.B + (size_t)(unsigned)j * a.ldb + c0));
+  };
+#pragma unroll 1
+  for (int r = t >> 3; r < kBandRows; r += kSpmmCta / 8) {
+    if (i0 + r >= M) return;
+    float s[8];
+    auto add = [&](float x, const uint4 &g) {
+      const uint32_t wd[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        s[2 * q] = fmaf(x, bf16lo(wd[q]), s[2 * q]);
+        s[2 * q + 1] = fmaf(x, bf16hi(wd[q]), s[2 * q + 1]);
+      }
+    };
+    const int n = cnt[r];
+    if (direct) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) s[q] = 0.0f;
+      for (int k = rp[r]; k < rp[r + 1]; ++k) add(ld_val(a.val, k), gather(__ldg(a.col + k)));
+    } else {
+      const float *p0 = sums + r * (kBandCols + kBandCPad) + 8 * l;
+      const float *p1 = p0 + kBandRows * (kBandCols + kBandCPad);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) s[q] = p0[q] + p1[q];
+      if (n <= kBandList) {
+        for (int e0 = 0; e0 < n; e0 += 8) {
+          uint4 g[8];
+          float x[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const int2 it = list[r * kBandList + (e0 + e < n ? e0 + e : e0)];
+            g[e] = gather(it.x);
+            x[e] = __int_as_float(it.y);
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (e0 + e < n) add(x[e], g[e]);
+        }
+      } else {
+        // more off-band nonzeros than the list holds: walk the row
+        for (int k = rp[r]; k < rp[r + 1]; ++k) {
+          const int j = __ldg(a.col + k);
+          if ((unsigned)(j - jw0) >= (unsigned)win) add(ld_val(a.val, k), gather(j));
+        }
+      }
+    }
+    float *dst = a.C + (long long)(i0 + r) * a.ldc + c0;
+    __stcs(reinterpret_cast<float4 *>(dst), make_float4(s[0], s[1], s[2], s[3]));
+    __stcs(reinterpret_cast<float4 *>(dst) + 1, make_float4(s[4], s[5], s[6], s[7]));
   }
 }
 
@@ -409,8 +648,11 @@ template <typename BT> int launch_window(const SpmmLaunch &L, cudaStream_t s) {
   return set_error(SEGTACO_EUNSUPPORTED, "window: no variant V=%d G=%d", L.V, L.G);
 }
 
+// The band kernels: fp32 B with multiply-adds, bf16 B on the tensor cores (its
+// window in the 128-byte swizzle, rows rounded up to whole 16-row steps).
 template <typename BT> int launch_band_typed(const SpmmLaunch &L, cudaStream_t s) {
-  const int win = kBandRows + 2 * L.band_halo;
+  constexpr bool kMma = sizeof(BT) == 2;
+  const int win = kMma ? band_mma_win(L.band_halo) : kBandRows + 2 * L.band_halo;
   if (L.band_halo < 0 || win > 256)
     return set_error(SEGTACO_EINVAL, "band window of %d rows (32 + 2*halo) > 256", win);
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
@@ -423,12 +665,20 @@ template <typename BT> int launch_band_typed(const SpmmLaunch &L, cudaStream_t s
   const CUresult r = enc(&tm, sizeof(BT) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                                : CU_TENSOR_MAP_DATA_TYPE_UINT16,
                          2, const_cast<void *>(L.B), dims, strides, box, es,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         kMma ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     return set_error(SEGTACO_EINVAL, "band: tensor map of B rejected (CUresult %d)", (int)r);
-  const size_t bytes = band_smem<BT>(win).bytes;
-  auto kern = spmm_band_kernel<BT>;
+  void (*kern)(SpmmArgs<BT>, const CUtensorMap, int, int *);
+  size_t bytes;
+  if constexpr (kMma) {
+    kern = spmm_band_mma_kernel;
+    bytes = band_mma_smem(win).bytes;
+  } else {
+    kern = spmm_band_kernel;
+    bytes = band_smem(win).bytes;
+  }
   static std::atomic<unsigned long long> opted{0};
   int dev = 0;
   SEGTACO_TRY(check_cuda(cudaGetDevice(&dev), "cudaGetDevice"));
