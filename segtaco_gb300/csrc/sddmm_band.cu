@@ -5,20 +5,34 @@
 // bytes for D = 64 fp32) and keep X[i] in registers while a row lasts; on a
 // banded matrix those gathers hit L1 and the load/store data pipe bounds them.
 // Rows i and i + 1 share almost all of their band, so here a CTA owns 32
-// consecutive rows and computes every dot product of its band at once: it
-// stages the rows' X block (32 x D) and the Y window of 32 + 2 kSbHalo rows
-// around the diagonal (column i0 * K / M of its first row) in shared memory,
-// both transposed (d-major), and each thread forms a 4 x 6 block of the dense
-// tile <X[4rb + q], Y[jw0 + 6cb + c]> with 4 shared loads per step of d for
-// 24 multiply-adds.  The tile then goes to shared memory and every nonzero of
-// the block reads its dot product there.  Nonzeros outside the window (off
-// band) are listed (kSbList per block) and then computed by 16 lanes each, 4
-// elements per lane from a row-major copy of the X block and Y[j] in global
-// memory, summed by shuffles; beyond the list a thread computes the dot
-// product alone.  The tile holds dot products for window positions without a
-// nonzero too (96 per row instead of ~2 kSbHalo + 1).
+// consecutive rows and computes every dot product of its band at once: the dense
+// tile <X[i0 + r], Y[jw0 + j]> of its 32 rows and the 32 + 2 kSbHalo window rows
+// around the diagonal (column i0 * K / M of its first row), a 32 x 96 x 64
+// contraction that runs as mma.m16n8k16 with fp32 accumulation.  bf16 factors take one
+// product per step.  fp32 factors are cut exactly into three bf16 parts (hi + mid +
+// lo, 8 bits each) and the six products down to 2^-16 of the largest are summed per
+// step of 16 elements, the smallest first, then added to the running sum in fp32; what
+// is left out is below 2^-24 of a product.  Warp w takes window rows 24 w .. +23 and
+// all 32 rows; a lane's four elements of a row are one load of 16 (8) bytes, in the
+// same order for X and Y, so neither needs transposing or, for Y, shared memory.  The
+// tile then goes to shared memory and every nonzero of the block reads its dot product
+// there.  Nonzeros outside the window (off band) are listed (kSbList per block) and then
+// computed by 16 lanes each, 4 elements per lane from the X block and Y[j] in global
+// memory, summed by shuffles; beyond the list a thread computes the dot product alone.
+// The tile holds dot products for window positions without a nonzero too (96 per row
+// instead of ~2 kSbHalo + 1).  Splitting an infinity or NaN would make NaN of both: a
+// CTA that meets one in fp32 factors computes its dot products one by one instead.
+//
+// What bounds it: the sampling of the tile and the off-band gathers, each about half
+// of what the product leaves (without the off-band list 136 us, without the product
+// 158).  Measured on GB300, banded-plus-random 262,144 rows, half band 32, 8 off-band
+// nonzeros per row, multiply-adds on 4 x 6 register tiles -> here: fp32 246 -> 194 us,
+// bf16 222 -> 150; error against FP64 1.4e-7 -> 9.7e-8 and 5.0e-8 -> 4.6e-8.  Eight
+// off-band steps in flight instead of four 206 -> 195 us; 20 sampled nonzeros in flight
+// instead of 10 spill (258); a warp per row in the sampling 252.
 #include "common.cuh"
 #include "internal.h"
+#include "mma.cuh"
 
 namespace segtaco {
 namespace {
@@ -27,14 +41,11 @@ constexpr int kSbRows = 32;                     // rows per CTA
 constexpr int kSbHalo = 32;                     // window rows on either side
 constexpr int kSbWin = kSbRows + 2 * kSbHalo;  // 96 window rows
 constexpr int kSbD = 64;                        // dot-product length
-// Pitches (floats) of the transposed X block and Y window: 16-byte rows for X
-// (a thread reads its 4 rows with one 16-byte load), 8-byte rows for Y whose
-// 6-column reads of 16 threads cover 32 distinct banks.
-constexpr int kSbXP = kSbRows + 4;
-constexpr int kSbYP = kSbWin + 2;
+constexpr int kSbTP = kSbWin + 8;  // pitch of the tile: conflict-free 8-byte stores
+constexpr int kSbXP = kSbD + 16;   // pitch of the X block: conflict-free 16-byte loads
 constexpr int kSbCta = 128;
+constexpr int kSq = 10;       // nonzeros in flight per thread of the sampling pass
 constexpr int kSbList = 512;  // off-band nonzeros listed per block
-constexpr int kSbXR = kSbD + 4;  // pitch of the row-major X copy (floats)
 
 // Four consecutive X or Y values as floats (fp32: 16 bytes; bf16: 8 bytes).
 template <typename XT> __device__ __forceinline__ float4 sb_ld4(const XT *p) {
@@ -45,130 +56,154 @@ template <typename XT> __device__ __forceinline__ float4 sb_ld4(const XT *p) {
     return make_float4(bf16lo(x.x), bf16hi(x.x), bf16lo(x.y), bf16hi(x.y));
   }
 }
+// Two floats as a bf16 pair (exact for values that are bf16).
+__device__ __forceinline__ uint32_t sb_pair(float x, float y) {
+  return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+}
 
 template <typename XT>
-__global__ void __launch_bounds__(kSbCta, 6)  // 34.4 KB of shared memory: six per SM
+__global__ void __launch_bounds__(kSbCta, sizeof(XT) == 4 ? 5 : 6)  // 96 / 80 registers
     sddmm_band_kernel(int M, int K, const int *__restrict__ row_ptr, const int *__restrict__ col,
                       const float *__restrict__ val, const XT *__restrict__ X,
                       const XT *__restrict__ Y, long long ldx, long long ldy,
                       float *__restrict__ out) {
-  __shared__ __align__(16) float xt[kSbD * kSbXP];  // xt[d][r]
-  __shared__ __align__(16) float yt[kSbD * kSbYP];  // yt[d][jr]; later the tile [r][jr]
+  constexpr bool kSplit = sizeof(XT) == 4;
+  constexpr int kParts = kSplit ? 3 : 1;
+  __shared__ __align__(16) float xr[kSbRows * kSbXP];    // X block, row-major
+  __shared__ __align__(16) float tile[kSbRows * kSbTP];  // tile[r][window row]
+  __shared__ int4 lst[kSbList];                          // (k, row, column, value bits)
   __shared__ int rp[kSbRows + 1];
   __shared__ int lcount;
-  // Off-band nonzeros (k, row, column, value bits), in the X block's space once
-  // the tile product no longer reads it.
-  static_assert(kSbList * 4 <= kSbD * kSbXP, "the list fits the transposed X block");
-  int4 *lst = reinterpret_cast<int4 *>(xt);
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const int i0 = blockIdx.x * kSbRows;
   const int jw0 = (int)((long long)i0 * K / M) - kSbHalo;
-  // X block and Y window, transposed; rows outside [0, M) / [0, K) are zeros.
-  // Every thread loads its 4 X and 12 Y vectors, four at a time, before it
-  // stores them.
-  static_assert(kSbRows * (kSbD / 4) == 4 * kSbCta && kSbWin * (kSbD / 4) == 12 * kSbCta,
-                "staging shape");
-  constexpr int kSv = 8;  // vectors in flight per thread
+  // Y: lane g = lane / 4 of n-tile n holds window row 24 w + 8 n + g, elements
+  // 16 s + 4 (lane % 4) .. +3 in step s; rows outside [0, K) are zeros.
+  const int e4 = 4 * (lane & 3);
+  const XT *yrow[3];
+  bool yok[3];
 #pragma unroll
-  for (int pass = 0; pass < 16 / kSv; ++pass) {
-    float4 v[kSv];
-#pragma unroll
-    for (int u = 0; u < kSv; ++u) {
-      const int e = t + (pass * kSv + u) * kSbCta;  // 0 .. 511: X, 512 .. 2047: Y
-      if (e < kSbRows * (kSbD / 4)) {
-        const int i = i0 + e / (kSbD / 4);
-        v[u] = i < M ? sb_ld4<XT>(X + (size_t)i * ldx + 4 * (e % (kSbD / 4)))
-                     : make_float4(0, 0, 0, 0);
-      } else {
-        const int e2 = e - kSbRows * (kSbD / 4);
-        const int j = jw0 + e2 / (kSbD / 4);
-        v[u] = j >= 0 && j < K ? sb_ld4<XT>(Y + (size_t)j * ldy + 4 * (e2 % (kSbD / 4)))
-                               : make_float4(0, 0, 0, 0);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kSv; ++u) {
-      const int e = t + (pass * kSv + u) * kSbCta;
-      float *dst;
-      int pitch, col, q;
-      if (e < kSbRows * (kSbD / 4)) {
-        dst = xt, pitch = kSbXP, col = e / (kSbD / 4), q = e % (kSbD / 4);
-      } else {
-        const int e2 = e - kSbRows * (kSbD / 4);
-        dst = yt, pitch = kSbYP, col = e2 / (kSbD / 4), q = e2 % (kSbD / 4);
-      }
-      dst[(4 * q + 0) * pitch + col] = v[u].x;
-      dst[(4 * q + 1) * pitch + col] = v[u].y;
-      dst[(4 * q + 2) * pitch + col] = v[u].z;
-      dst[(4 * q + 3) * pitch + col] = v[u].w;
-    }
+  for (int n = 0; n < 3; ++n) {
+    const int j = jw0 + 24 * w + 8 * n + (lane >> 2);
+    yok[n] = j >= 0 && j < K;
+    yrow[n] = Y + (size_t)(yok[n] ? j : 0) * ldy + e4;
   }
-  if (t <= kSbRows) rp[t] = __ldg(row_ptr + min(i0 + t, M));
-  if (t == 0) lcount = 0;
-  __syncthreads();
-  // The dense tile: rows 4rb .. 4rb+3 x window rows 6cb .. 6cb+5.
-  const int rb = t >> 4, cb = t & 15;
-  float acc[4][6];
+  auto load_y = [&](int s, float4(&y)[3]) {
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int c = 0; c < 6; ++c) acc[q][c] = 0.0f;
-#pragma unroll 4
-  for (int d = 0; d < kSbD; ++d) {
-    const float4 x4 = *reinterpret_cast<const float4 *>(xt + d * kSbXP + 4 * rb);
-    const float x[4] = {x4.x, x4.y, x4.z, x4.w};
-    float y[6];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const float2 y2 = *reinterpret_cast<const float2 *>(yt + d * kSbYP + 6 * cb + 2 * c);
-      y[2 * c] = y2.x;
-      y[2 * c + 1] = y2.y;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int c = 0; c < 6; ++c) acc[q][c] = fmaf(x[q], y[c], acc[q][c]);
-  }
-  __syncthreads();  // every thread is done with yt
-  float *tile = yt;  // tile[r][jr], pitch kSbYP
-  float *xr = yt + kSbRows * kSbYP;  // X block row-major, pitch kSbXR (after the tile)
-  static_assert(kSbRows * kSbYP + kSbRows * kSbXR <= kSbD * kSbYP, "tile and X copy fit");
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int c = 0; c < 6; ++c) tile[(4 * rb + q) * kSbYP + 6 * cb + c] = acc[q][c];
+    for (int n = 0; n < 3; ++n)
+      y[n] = yok[n] ? sb_ld4<XT>(yrow[n] + 16 * s) : make_float4(0, 0, 0, 0);
+  };
+  float4 ycur[3];
+  load_y(0, ycur);
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const int e = t + u * kSbCta;  // 0 .. 511: row e / 16, elements 4 (e % 16) ..
     const int i = i0 + e / (kSbD / 4);
-    const float4 x = i < M ? sb_ld4<XT>(X + (size_t)i * ldx + 4 * (e % (kSbD / 4)))
-                           : make_float4(0, 0, 0, 0);
-    *reinterpret_cast<float4 *>(xr + (e / (kSbD / 4)) * kSbXR + 4 * (e % (kSbD / 4))) = x;
+    *reinterpret_cast<float4 *>(xr + (e / (kSbD / 4)) * kSbXP + 4 * (e % (kSbD / 4))) =
+        i < M ? sb_ld4<XT>(X + (size_t)i * ldx + 4 * (e % (kSbD / 4))) : make_float4(0, 0, 0, 0);
   }
+  if (t <= kSbRows) rp[t] = __ldg(row_ptr + min(i0 + t, M));
+  if (t == 0) lcount = 0;
   __syncthreads();
-  // The block's nonzeros, coalesced, eight per thread per pass.
-  constexpr int SQ = 8;
-  const int k_end = rp[kSbRows];
-  for (int k0 = rp[0] + t; k0 < k_end; k0 += SQ * kSbCta) {
-    int cj[SQ];
-    float cv[SQ];
+  // ---- the dense tile ----
+  float acc[2][3][4];
 #pragma unroll
-    for (int u = 0; u < SQ; ++u) {
-      const int k = k0 + u * kSbCta;
-      cj[u] = k < k_end ? __ldg(col + k) : 0;
-      cv[u] = k < k_end ? (val ? __ldg(val + k) : 1.0f) : 0.0f;
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < 3; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.0f;
+  float amax = 0.0f;  // the factors' largest magnitude, or NaN
+#pragma unroll 1
+  for (int s = 0; s < kSbD / 16; ++s) {
+    float4 ynext[3];
+    if (s + 1 < kSbD / 16) load_y(s + 1, ynext);
+    uint32_t xa[2][kParts][4];  // [m-tile][part][register]
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {  // rows g, g + 8, g + 16, g + 24
+      const float4 x = *reinterpret_cast<const float4 *>(xr + (8 * h + (lane >> 2)) * kSbXP +
+                                                         16 * s + e4);
+      uint32_t(&p)[kParts][4] = xa[h >> 1];
+      const int q = h & 1;  // registers q (elements 0, 1) and q + 2 (elements 2, 3)
+      if constexpr (kSplit) {
+        amax = max_nan(max_nan(max_nan(max_nan(amax, x.x), x.y), x.z), x.w);
+        split3(x.x, x.y, p[0][q], p[1][q], p[2][q]);
+        split3(x.z, x.w, p[0][q + 2], p[1][q + 2], p[2][q + 2]);
+      } else {
+        p[0][q] = sb_pair(x.x, x.y);
+        p[0][q + 2] = sb_pair(x.z, x.w);
+      }
     }
 #pragma unroll
-    for (int u = 0; u < SQ; ++u) {
-      const int k = k0 + u * kSbCta;
-      if (k < k_end) {
-        int r = 0;  // the last row whose start is <= k
+    for (int n = 0; n < 3; ++n) {
+      uint32_t yb[kParts][2];
+      const float4 y = ycur[n];
+      if constexpr (kSplit) {
+        amax = max_nan(max_nan(max_nan(max_nan(amax, y.x), y.y), y.z), y.w);
+        split3(y.x, y.y, yb[0][0], yb[1][0], yb[2][0]);
+        split3(y.z, y.w, yb[0][1], yb[1][1], yb[2][1]);
+      } else {
+        yb[0][0] = sb_pair(y.x, y.y);
+        yb[0][1] = sb_pair(y.z, y.w);
+      }
 #pragma unroll
-        for (int step = 16; step > 0; step >>= 1)
-          if (r + step <= kSbRows - 1 && rp[r + step] <= k) r += step;
+      for (int m = 0; m < 2; ++m) {
+        float d[4];
+        if constexpr (kSplit) {
+          mma_bf16_zero(d, xa[m][0], yb[2][0], yb[2][1]);  // hi lo
+          mma_bf16(d, xa[m][2], yb[0][0], yb[0][1]);       // lo hi
+          mma_bf16(d, xa[m][1], yb[1][0], yb[1][1]);       // mid mid
+          mma_bf16(d, xa[m][0], yb[1][0], yb[1][1]);       // hi mid
+          mma_bf16(d, xa[m][1], yb[0][0], yb[0][1]);       // mid hi
+          mma_bf16(d, xa[m][0], yb[0][0], yb[0][1]);       // hi hi
+        } else {
+          mma_bf16_zero(d, xa[m][0], yb[0][0], yb[0][1]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[m][n][q] += d[q];
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 3; ++n) ycur[n] = ynext[n];
+  }
+  constexpr int SQ = kSq;
+  const int k_beg = rp[0], len = rp[kSbRows] - k_beg;
+  int cj[SQ];
+  float cv[SQ];
+  auto load_nz = [&](int n0) {
+#pragma unroll
+    for (int u = 0; u < SQ; ++u) {
+      const bool has = n0 + u * kSbCta < len;
+      cj[u] = has ? __ldg(col + (k_beg + n0 + u * kSbCta)) : 0;
+      cv[u] = has && val ? __ldg(val + (k_beg + n0 + u * kSbCta)) : 1.0f;
+    }
+  };
+  load_nz(t);
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+      float *dst = tile + (16 * m + (lane >> 2)) * kSbTP + 24 * w + 8 * n + 2 * (lane & 3);
+      *reinterpret_cast<float2 *>(dst) = make_float2(acc[m][n][0], acc[m][n][1]);
+      *reinterpret_cast<float2 *>(dst + 8 * kSbTP) = make_float2(acc[m][n][2], acc[m][n][3]);
+    }
+  // An infinity or NaN among fp32 factors: every dot product by itself.
+  const bool direct = __syncthreads_or(kSplit && !(fabsf(amax) <= 3.402823466e38f)) != 0;
+  // The block's nonzeros, coalesced, kSq per thread per pass.
+  for (int n0 = t; n0 < len; n0 += SQ * kSbCta) {
+    if (n0 != t) load_nz(n0);
+    int r = 0;  // the last row whose start is <= the thread's first nonzero
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (r + step <= kSbRows - 1 && rp[r + step] - k_beg <= n0) r += step;
+    int rend = rp[r + 1] - k_beg;
+#pragma unroll
+    for (int u = 0; u < SQ; ++u) {
+      const int n = n0 + u * kSbCta;
+      if (n < len) {
+        while (n >= rend) rend = rp[++r + 1] - k_beg;  // n < rp[kSbRows] - k_beg
+        const int k = k_beg + n;
         const unsigned dj = (unsigned)(cj[u] - jw0);
-        if (dj < (unsigned)kSbWin) {
-          out[k] = cv[u] * tile[r * kSbYP + dj];
+        if (dj < (unsigned)kSbWin && !direct) {
+          out[k] = cv[u] * tile[r * kSbTP + dj];
         } else {
           const int slot = atomicAdd(&lcount, 1);
           if (slot < kSbList) {
@@ -176,17 +211,17 @@ __global__ void __launch_bounds__(kSbCta, 6)  // 34.4 KB of shared memory: six p
           } else {
             // past the list: the dot product by this thread alone
             const XT *yr = Y + (size_t)(unsigned)cj[u] * ldy;
-            float s = 0.0f;
+            float sum = 0.0f;
 #pragma unroll 4
             for (int q = 0; q < kSbD / 4; ++q) {
               const float4 y = sb_ld4<XT>(yr + 4 * q);
-              const float4 x = *reinterpret_cast<const float4 *>(xr + r * kSbXR + 4 * q);
-              s = fmaf(x.x, y.x, s);
-              s = fmaf(x.y, y.y, s);
-              s = fmaf(x.z, y.z, s);
-              s = fmaf(x.w, y.w, s);
+              const float4 x = *reinterpret_cast<const float4 *>(xr + r * kSbXP + 4 * q);
+              sum = fmaf(x.x, y.x, sum);
+              sum = fmaf(x.y, y.y, sum);
+              sum = fmaf(x.z, y.z, sum);
+              sum = fmaf(x.w, y.w, sum);
             }
-            out[k] = cv[u] * s;
+            out[k] = cv[u] * sum;
           }
         }
       }
@@ -194,11 +229,11 @@ __global__ void __launch_bounds__(kSbCta, 6)  // 34.4 KB of shared memory: six p
   }
   __syncthreads();
   // Listed off-band nonzeros: 16 lanes each (lane l: elements 4l .. 4l+3); a
-  // warp takes two per step, four steps with their gathers in flight at once,
+  // warp takes two per step, eight steps with their gathers in flight at once,
   // and every lane of it takes part in the shuffles.
   const int n = min(lcount, kSbList);
-  const int w = t >> 5, hw = (t >> 4) & 1, l = t & 15;
-  constexpr int kSteps = 4, kStride = kSbCta / 16;  // 8 entries per step over the CTA
+  const int hw = (t >> 4) & 1, l = t & 15;
+  constexpr int kSteps = 8, kStride = kSbCta / 16;  // 8 entries per step over the CTA
   for (int e0 = 2 * w; e0 < n; e0 += kSteps * kStride) {
     int4 it[kSteps];
     float4 y[kSteps];
@@ -210,7 +245,7 @@ __global__ void __launch_bounds__(kSbCta, 6)  // 34.4 KB of shared memory: six p
     }
 #pragma unroll
     for (int u = 0; u < kSteps; ++u) {
-      const float4 x = *reinterpret_cast<const float4 *>(xr + it[u].y * kSbXR + 4 * l);
+      const float4 x = *reinterpret_cast<const float4 *>(xr + it[u].y * kSbXP + 4 * l);
       float s = x.x * y[u].x;
       s = fmaf(x.y, y[u].y, s);
       s = fmaf(x.z, y[u].z, s);
