@@ -116,6 +116,14 @@ void *Scratch::take(size_t bytes) {
 // ---------------------------------------------------------------------------
 static bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
+// Products of at most this many elements of C search their chunk edges in the split
+// walk's kernel and clear C whole, instead of running the partition kernel: one
+// launch and no scratch.  Measured on GB300, partition / search, device time of a
+// call: 1000 lognormal rows, N = 16 7.8 / 5.9 us; 10,000, N = 61 18.3 / 9.8; 28,000, N =
+// 128 (3.6M elements) 23.6 / 21.9; 200,000 power-law rows, N = 16 (3.2M) 39.9 / 41.4;
+// 77,777 rows, N = 128 (10M) 38.2 / 43.2.  An untuned call of 1000 rows from Python 15.5
+// -> 10.3 us without the scratch.
+constexpr long long kSearchMaxElems = 2LL << 20;
 // Merge-path chunks up to this many items take the split walk (a warp stages
 // its chunk in shared memory).
 constexpr long long kSplitMaxItems = 512;
@@ -427,7 +435,12 @@ int run_spmm_planned(const SpmmPlan &plan, int M, int K, long long nnz, const in
       return bf16 ? launch_spmm_bf16_rows(L, s) : launch_spmm_f32_rows(L, s);
     case SEGTACO_EB_SR:
     case SEGTACO_EB_PR:
-      if (!partition_ready)
+      if (px == nullptr)  // no partition arrays: rows cut by a chunk edge are added to zeros
+        SEGTACO_TRY(check_cuda(
+            ldc == N ? cudaMemsetAsync(C, 0, (size_t)M * N * sizeof(float), s)
+                     : cudaMemset2DAsync(C, ldc * sizeof(float), 0, N * sizeof(float), M, s),
+            "clearing C"));
+      else if (!partition_ready)
         SEGTACO_TRY(launch_merge_path(row_ptr, M, nnz, plan.items_per_unit, plan.nchunks, px, py,
                                       C, ldc, N, s));
       if (L.use_tma) return bf16 ? launch_spmm_tma_bf16(L, false, s) : launch_spmm_tma_f32(L, false, s);
@@ -638,14 +651,16 @@ int segtaco_spmm(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr, cons
   SpmmPlan plan;
   SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, ldb, ldc, B, C, cfg, &plan));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const bool ready = cfg && (cfg->flags & SEGTACO_FLAG_PARTITION_READY);
+  const bool search = !ready && plan.walk == 5 && (long long)M * N <= kSearchMaxElems;
   Scratch scratch(workspace, workspace_bytes, s);
-  SEGTACO_TRY(scratch.reserve(plan.workspace));
+  if (workspace || !search)  // (a caller's workspace is checked, if not needed)
+    SEGTACO_TRY(scratch.reserve(plan.workspace));
   int *px = nullptr, *py = nullptr;
-  if (plan.workspace) {
+  if (plan.workspace && !search) {
     px = static_cast<int *>(scratch.take(plan.px_entries * sizeof(int)));
     py = static_cast<int *>(scratch.take(plan.py_entries * sizeof(int)));
   }
-  const bool ready = cfg && (cfg->flags & SEGTACO_FLAG_PARTITION_READY);
   if (ready && plan.workspace && !workspace)
     return set_error(SEGTACO_EINVAL, "PARTITION_READY needs the caller's workspace");
   return run_spmm_planned(plan, M, K, nnz, row_ptr, col, vals, B, b_dtype, ldb, C, ldc, N, px, py,

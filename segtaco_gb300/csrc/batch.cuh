@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kSpmmCta, split_min_ctas<BT, E, C, G>())
     const long long local = (long long)item - bp.item_begin;
     const long long units = bp.a.units;
     const int slab = (int)(local / units);
-    spmm_split_unit<BT, E, C, G>(bp.a, local - (long long)slab * units, slab, lane, D,
+    spmm_split_unit<BT, E, C, G>(bp.a, chunk_edges(bp.a, local - (long long)slab * units), slab, lane, D,
                                  split_sm + threadIdx.x / 32 * split_words<E * C>(D));
     __syncwarp();  // the staging is free for the next item
   }

@@ -450,8 +450,8 @@ __device__ __forceinline__ void merge_path_store_row(const int *__restrict__ row
     if ((long long)__ldg(row_ptr + r) < dl - r) {  // y grows with c: test the last edge
       float *dst = C + r * ldc;
       int k = 0;
-      if ((((uintptr_t)dst) & 15) == 0)
-        for (; k + 4 <= N; k += 4) *reinterpret_cast<float4 *>(dst + k) = make_float4(0, 0, 0, 0);
+      for (; k < N && (((uintptr_t)(dst + k)) & 15) != 0; ++k) dst[k] = 0.0f;
+      for (; k + 4 <= N; k += 4) *reinterpret_cast<float4 *>(dst + k) = make_float4(0, 0, 0, 0);
       for (; k < N; ++k) dst[k] = 0.0f;
     }
   }

@@ -60,9 +60,50 @@ template <int V> __host__ __device__ inline int split_words(int D) {
   return split_head<V>(D) + 32 * V;
 }
 
+// Edges of a chunk: row and nonzero coordinates of its first and last merge item.
+struct ChunkEdges {
+  int x0, y0, x1, y1;
+};
+template <typename BT>
+__device__ __forceinline__ ChunkEdges chunk_edges(const SpmmArgs<BT> &a, long long w) {
+  return {__ldg(a.part_x + w), __ldg(a.part_y + w), __ldg(a.part_x + w + 1),
+          __ldg(a.part_y + w + 1)};
+}
+// The same without partition arrays: lanes 0-15 search the chunk's first diagonal,
+// lanes 16-31 its last, 16 probes a round (the row coordinate is the number of row
+// ends r with row_ptr[r + 1] + r + 1 <= d, as in merge_path_x).
+template <typename BT>
+__device__ __forceinline__ ChunkEdges search_edges(const SpmmArgs<BT> &a, long long w, int D,
+                                                  int lane) {
+  const unsigned FULL = 0xffffffffu;
+  const int l = lane & 15;
+  const long long total = (long long)a.M + a.nnz;
+  long long d = (w + (lane >> 4)) * (long long)D;
+  if (d > total) d = total;
+  long long lo = d > a.nnz ? d - a.nnz : 0, hi = d < a.M ? d : a.M;  // lo <= x <= hi
+  while (__any_sync(FULL, lo < hi)) {
+    // row ends lo .. hi-1 are open; probe l asks for row lo + (l + 1) step - 1
+    const long long step = (hi - lo + 15) / 16;
+    const long long at = lo + (l + 1) * step - 1;
+    const bool past = at >= hi || (long long)__ldg(a.row_ptr + at + 1) + at + 1 > d;
+    const unsigned m = (__ballot_sync(FULL, past) >> (lane & 16)) & 0xffffu;
+    if (lo < hi) {
+      const int f = m ? __ffs(m) - 1 : 16;  // probes 0 .. f-1 have ended
+      const long long nhi = lo + (f + 1) * step - 1;
+      lo += f * step;
+      if (lo > hi) lo = hi;
+      if (f < 16 && nhi < hi) hi = nhi;
+    }
+  }
+  const int x = (int)lo, y = (int)(d - lo);
+  return {__shfl_sync(FULL, x, 0), __shfl_sync(FULL, y, 0), __shfl_sync(FULL, x, 16),
+          __shfl_sync(FULL, y, 16)};
+}
+
 template <typename BT, int E, int C, int G>
-__device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, long long w, int slab,
-                                                int lane, int D, int *__restrict__ sm) {
+__device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, const ChunkEdges ce,
+                                                int slab, int lane, int D,
+                                                int *__restrict__ sm) {
   constexpr int P = 32 / G;
   constexpr int V = E * C;
   constexpr int S = kSplitStep;
@@ -85,8 +126,7 @@ __device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, long long
   char *Cc = reinterpret_cast<char *>(a.C + col0);
   const unsigned ldc = (unsigned)a.ldc * 4u;
 
-  const int x0 = __ldg(a.part_x + w), y0 = __ldg(a.part_y + w);
-  const int x1 = __ldg(a.part_x + w + 1), y1 = __ldg(a.part_y + w + 1);
+  const int x0 = ce.x0, y0 = ce.y0, x1 = ce.x1, y1 = ce.y1;
   const int rp0 = x0 < M ? __ldg(a.row_ptr + x0) : y0;
   // Row x0 began in an earlier chunk; row x1 holds nonzeros here and ends later.
   const bool head_split = rp0 < y0;
@@ -259,13 +299,16 @@ template <typename BT, int E, int C, int G> constexpr int split_min_ctas() {
   return (E * C * sizeof(BT) > 16 || C > 1 ? 32 : 36) / kSpmmWarps;
 }
 
+// a.part_x null: the chunk's edges are searched here and C is zero on entry.
 template <typename BT, int E, int C, int G>
 __global__ void __launch_bounds__(kSpmmCta, split_min_ctas<BT, E, C, G>())
     spmm_split_kernel(SpmmArgs<BT> a, int D) {
   extern __shared__ __align__(16) int split_sm[];
   const long long w = (long long)blockIdx.x * kSpmmWarps + threadIdx.x / 32;
   if (w >= a.units) return;  // whole warp leaves together
-  spmm_split_unit<BT, E, C, G>(a, w, blockIdx.y, threadIdx.x & 31, D,
+  const int lane = threadIdx.x & 31;
+  const ChunkEdges ce = a.part_x ? chunk_edges(a, w) : search_edges(a, w, D, lane);
+  spmm_split_unit<BT, E, C, G>(a, ce, blockIdx.y, lane, D,
                                split_sm + threadIdx.x / 32 * split_words<E * C>(D));
 }
 

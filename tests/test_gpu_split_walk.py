@@ -66,6 +66,27 @@ def test_unused_rows_of_b_do_not_reach_c(cuda, n):
         assert_spmm_close(_run(A, torch.from_numpy(bad).cuda(), cfg), A, B, ref=ref)
 
 
+@pytest.mark.parametrize("rows,n", [(1, 8), (2, 33), (700, 64), (16_384, 128), (16_385, 128)])
+def test_edges_searched_or_partitioned(cuda, rows, n):
+    """Up to 2M elements of C the kernel searches its chunk edges; with prepared partition arrays, and
+    past that, it reads them.  The same product, also into a strided C, with the padding left alone."""
+    A = synth.random_csr(rows, 300, 0.02, seed=rows, p_empty=0.2, long_rows={0: 250, rows - 1: 300})
+    B = synth.dense(A.K, n, seed=1)
+    ref = spmm_ref(A, B)
+    Ad, Bd = dev(A), torch.from_numpy(B).cuda()
+    cfg = N.Config.make(schedule="eb_sr")
+    ws = torch.empty(ops.spmm_workspace_size(Ad, n, N.F32, cfg), dtype=torch.uint8, device="cuda")
+    wide = torch.full((A.M, n + 4), 7.0, device="cuda")
+    for C in (torch.full((A.M, n), float("nan"), device="cuda"), wide[:, :n]):
+        ops.spmm(Ad, Bd, C, cfg)
+        assert_spmm_close(C.cpu().numpy(), A, B, ref=ref)
+        ops.spmm_partition(Ad, C, cfg, ws)
+        ready = N.Config.make(schedule="eb_sr", flags=N.FLAG_PARTITION_READY)
+        ops.spmm(Ad, Bd, C, ready, ws)
+        assert_spmm_close(C.cpu().numpy(), A, B, ref=ref)
+    assert (wide[:, n:] == 7.0).all()
+
+
 @pytest.mark.parametrize("n,pad,bf16", [(64, 0, False), (37, 0, False), (126, 0, True), (40, 4, True)])
 def test_batches_of_the_split_walk(cuda, n, pad, bf16):
     mats = list(CASES.values()) + [synth.random_csr(50, 60, 0.0, seed=9)]
