@@ -194,13 +194,15 @@ int need(const taco_tensor_t *t, const char *what, bool csr) {
 // Pipelined copies around the SpMM.  The call's time is mostly the link: the
 // operands go in and C comes out over host<->device copies.  The product is cut
 // into tiles of (column slab of B and C) x (row block of A and C):
-//   * wide N (a multiple of 32, at least 64): A goes in whole, then B one
-//     32-column slab at a time (2D copies); the tiles of slab s run as soon as
-//     slab s has landed, so C starts coming back while later slabs go in;
+//   * pinned B and C with wide N (a multiple of 32, at least 64): A goes in whole,
+//     then B one 32-column slab at a time (2D copies); the tiles of slab s run as
+//     soon as slab s has landed, so C starts coming back while later slabs go in;
 //   * otherwise one slab: B and row_ptr go in first, then A's nonzeros block by
 //     block, each block's tile running once its nonzeros have landed.
-// Each tile's rows and columns of C go back (a 2D copy) while the next tiles
-// compute.  A row block is a proper CSR of its own: its row_ptr is shifted to
+// Each tile's rows and columns of C go back while the next tiles compute.  Measured
+// on GB300 on pageable operands, column slabs before -> whole copies: 100,000
+// lognormal rows, N = 64 542 -> 434 us, N = 128 915 -> 754; 400,000 power-law rows, N =
+// 128 3.37 -> 2.88 ms; N = 42, K = 70,741 (one 2D copy before) 2159 -> 147 us.  A row block is a proper CSR of its own: its row_ptr is shifted to
 // start at 0 on the device and its col / vals pointers start at its first
 // nonzero.  Row blocks are balanced by rows + nonzeros.  The timer sums the
 // tiles' compute time (segTACO times {memset, partition, kernel} only,
@@ -255,15 +257,29 @@ int shim_streams(ShimStreams **out) {
   return SEGTACO_OK;
 }
 
+// Host memory the runtime does not know: its copies are over when the call returns
+// (H2D 167 GB/s, D2H 176 GB/s in whole copies; column slabs by 2D copies 140 and
+// 111), so the two directions never overlap and column slabs do not pay.
+bool pageable(const void *p) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return at.type == cudaMemoryTypeUnregistered;
+}
+
 int run_spmm_pipelined(const segtaco_config &cfg, int M, int K, long long nnz, const int *rp,
                        const int *col, const float *val, const float *Bh, int N, float *Ch,
                        DeviceCopies &dev) {
-  // Column slabs and row blocks (one per 32 MB of A's nonzeros and C).
-  int ns = (N >= 2 * kSlabCols && N % kSlabCols == 0) ? N / kSlabCols : 1;
+  // Column slabs (pinned operands) and row blocks (one per 32 MB of A's nonzeros and
+  // C; 16 MB where only the product overlaps the copies out).
+  const bool paged = pageable(Bh) || pageable(Ch);
+  int ns = (!paged && N >= 2 * kSlabCols && N % kSlabCols == 0) ? N / kSlabCols : 1;
   if (ns > kMaxSlabs) ns = 1;
   const int wcols = N / ns;
   const double bytes = (double)nnz * 8.0 + (double)M * N * 4.0;
-  int nb = (int)(bytes / (32.0 * (1 << 20))) / ns;
+  int nb = (int)(bytes / ((paged ? 16.0 : 32.0) * (1 << 20))) / ns;
   if (nb < 1) nb = 1;
   if (nb > kMaxBlocks) nb = kMaxBlocks;
   if (nb > M) nb = M > 0 ? M : 1;
@@ -313,19 +329,59 @@ int run_spmm_pipelined(const segtaco_config &cfg, int M, int K, long long nnz, c
     return rec(S->ready_a[b], S->in);
   };
   auto upload_slab = [&](int sl) {
-    if ((size_t)K * wcols)
+    // (a 2D copy of whole rows is not a plain copy to the runtime: 70,741 rows of 168
+    // bytes 2033 us, in one piece 72)
+    if (ns == 1)
+      SEGTACO_TRY(h2d(d_B, Bh, (size_t)K * N * 4));
+    else if ((size_t)K * wcols)
       SEGTACO_TRY(check_cuda(cudaMemcpy2DAsync((float *)d_B + sl * wcols, (size_t)N * 4,
                                                Bh + sl * wcols, (size_t)N * 4, (size_t)wcols * 4, K,
                                                cudaMemcpyHostToDevice, S->in),
                              "H2D slab"));
     return rec(S->ready_b[sl], S->in);
   };
-  // in
+  // compute: a block's row_ptr shifted to start at 0 (the only block's is as it is),
+  // and one tile
+  const bool shifted = nb > 1 || rp[0] != 0;
+  auto shift_rows = [&]() {
+    SEGTACO_TRY(check_cuda(cudaStreamWaitEvent(S->comp, S->ready_rp, 0), "cudaStreamWaitEvent"));
+    for (int b = 0; b < nb && shifted; ++b) {
+      const int r0 = rows[b], mb = rows[b + 1] - r0;
+      shift_rows_kernel<<<(mb + 1 + 255) / 256, 256, 0, S->comp>>>(
+          (const int *)d_rp + r0, (int *)d_rps + r0 + b, mb + 1, rp[r0]);
+      SEGTACO_TRY(check_launch("shift_rows_kernel"));
+    }
+    return SEGTACO_OK;
+  };
+  auto compute = [&](int sl, int b) {
+    const int t = sl * nb + b;
+    const int r0 = rows[b], mb = rows[b + 1] - r0;
+    const long long p0 = rp[r0], nnzb = rp[rows[b + 1]] - p0;
+    const int *block_rp = shifted ? (const int *)d_rps + r0 + b : (const int *)d_rp;
+    if (b == 0)
+      SEGTACO_TRY(check_cuda(cudaStreamWaitEvent(S->comp, S->ready_b[sl], 0),
+                             "cudaStreamWaitEvent"));
+    if (sl == 0)
+      SEGTACO_TRY(check_cuda(cudaStreamWaitEvent(S->comp, S->ready_a[b], 0),
+                             "cudaStreamWaitEvent"));
+    SEGTACO_TRY(rec(S->t0[t], S->comp));
+    SEGTACO_TRY(segtaco_spmm(mb, K, nnzb, block_rp, (const int *)d_col + p0,
+                             (const float *)d_val + p0, (const float *)d_B + sl * wcols,
+                             SEGTACO_F32, N, (float *)d_C + (long long)r0 * N + sl * wcols, N,
+                             wcols, &cfg, d_ws, ws, S->comp));
+    SEGTACO_TRY(rec(S->t1[t], S->comp));
+    return rec(S->done[t], S->comp);
+  };
+  // in, and the tiles as their operands land
   SEGTACO_TRY(h2d(d_rp, rp, (size_t)(M + 1) * 4));
   SEGTACO_TRY(rec(S->ready_rp, S->in));
   if (ns == 1) {
     SEGTACO_TRY(upload_slab(0));
-    for (int b = 0; b < nb; ++b) SEGTACO_TRY(upload_block(b));
+    SEGTACO_TRY(shift_rows());
+    for (int b = 0; b < nb; ++b) {
+      SEGTACO_TRY(upload_block(b));
+      SEGTACO_TRY(compute(0, b));
+    }
   } else {
     // Every tile waits for slab 0 of B, which follows A: A goes in as two
     // whole copies (fewer, larger copies: 4.84 -> 4.75 ms on the 1M x 1M
@@ -334,40 +390,20 @@ int run_spmm_pipelined(const segtaco_config &cfg, int M, int K, long long nnz, c
     SEGTACO_TRY(h2d(d_val, val, (size_t)nnz * 4));
     for (int b = 0; b < nb; ++b) SEGTACO_TRY(rec(S->ready_a[b], S->in));
     for (int sl = 0; sl < ns; ++sl) SEGTACO_TRY(upload_slab(sl));
-  }
-  // compute: shifted row_ptr of every block (once row_ptr is in), then the
-  // tiles slab by slab
-  SEGTACO_TRY(check_cuda(cudaStreamWaitEvent(S->comp, S->ready_rp, 0), "cudaStreamWaitEvent"));
-  for (int b = 0; b < nb; ++b) {
-    const int r0 = rows[b], mb = rows[b + 1] - r0;
-    shift_rows_kernel<<<(mb + 1 + 255) / 256, 256, 0, S->comp>>>(
-        (const int *)d_rp + r0, (int *)d_rps + r0 + b, mb + 1, rp[r0]);
-    SEGTACO_TRY(check_launch("shift_rows_kernel"));
-  }
-  for (int sl = 0; sl < ns; ++sl) {
-    SEGTACO_TRY(check_cuda(cudaStreamWaitEvent(S->comp, S->ready_b[sl], 0), "cudaStreamWaitEvent"));
-    for (int b = 0; b < nb; ++b) {
-      const int t = sl * nb + b;
-      const int r0 = rows[b], mb = rows[b + 1] - r0;
-      const long long p0 = rp[r0], nnzb = rp[rows[b + 1]] - p0;
-      if (sl == 0 || ns == 1)
-        SEGTACO_TRY(check_cuda(cudaStreamWaitEvent(S->comp, S->ready_a[b], 0),
-                               "cudaStreamWaitEvent"));
-      SEGTACO_TRY(rec(S->t0[t], S->comp));
-      SEGTACO_TRY(segtaco_spmm(mb, K, nnzb, (const int *)d_rps + r0 + b, (const int *)d_col + p0,
-                               (const float *)d_val + p0, (const float *)d_B + sl * wcols,
-                               SEGTACO_F32, N, (float *)d_C + (long long)r0 * N + sl * wcols, N,
-                               wcols, &cfg, d_ws, ws, S->comp));
-      SEGTACO_TRY(rec(S->t1[t], S->comp));
-      SEGTACO_TRY(rec(S->done[t], S->comp));
-    }
+    SEGTACO_TRY(shift_rows());
+    for (int sl = 0; sl < ns; ++sl)
+      for (int b = 0; b < nb; ++b) SEGTACO_TRY(compute(sl, b));
   }
   // out: each tile once computed
   for (int t = 0; t < ns * nb; ++t) {
     const int sl = t / nb, b = t % nb;
     const int r0 = rows[b], mb = rows[b + 1] - r0;
     SEGTACO_TRY(check_cuda(cudaStreamWaitEvent(S->out, S->done[t], 0), "cudaStreamWaitEvent"));
-    if ((size_t)mb * wcols)
+    if (ns == 1 && mb > 0)
+      SEGTACO_TRY(check_cuda(cudaMemcpyAsync(Ch + (long long)r0 * N, (float *)d_C + (long long)r0 * N,
+                                             (size_t)mb * N * 4, cudaMemcpyDeviceToHost, S->out),
+                             "D2H block"));
+    else if ((size_t)mb * wcols)
       SEGTACO_TRY(check_cuda(cudaMemcpy2DAsync(Ch + (long long)r0 * N + sl * wcols, (size_t)N * 4,
                                                (float *)d_C + (long long)r0 * N + sl * wcols,
                                                (size_t)N * 4, (size_t)wcols * 4, mb,
