@@ -741,11 +741,8 @@ int segtaco_csr_validate(int32_t M, int32_t K, int64_t nnz, const int32_t *row_p
   return SEGTACO_OK;
 }
 
-// SpMV is the N = 1 point of the SpMM segment kernel: eb_pr with one lane per
-// slot (32 nonzeros or short rows per warp step) over 512-item merge-path
-// chunks.  Measured on GB300 (1M x 1M power-law, 20.6M nonzeros): 0.140 ms,
-// against 0.222 ms for a dedicated merge-path tile kernel staging products in
-// shared memory.
+// The workspace that segtaco_spmv accepts: the partition of 512-item merge-path
+// chunks (spmv.cu needs none).
 static segtaco_config spmv_config() {
   segtaco_config c = {};
   c.schedule = SEGTACO_EB_PR;
@@ -772,19 +769,14 @@ int segtaco_spmv(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr, cons
   SEGTACO_TRY(check_csr_args(M, K, nnz, row_ptr, col));
   if (M == 0) return SEGTACO_OK;
   if (y == nullptr || (nnz > 0 && x == nullptr)) return set_error(SEGTACO_EINVAL, "x/y is NULL");
-  const segtaco_config c = spmv_config();
-  SpmmPlan plan;
-  SEGTACO_TRY(plan_spmm(M, K, nnz, 1, SEGTACO_F32, 1, 1, x, y, &c, &plan));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  Scratch scratch(workspace, workspace_bytes, s);
-  SEGTACO_TRY(scratch.reserve(plan.workspace));
-  int *px = nullptr, *py = nullptr;
-  if (plan.workspace) {
-    px = static_cast<int *>(scratch.take(plan.px_entries * sizeof(int)));
-    py = static_cast<int *>(scratch.take(plan.py_entries * sizeof(int)));
+  if (workspace) {  // checked, if no longer needed
+    size_t need = 0;
+    SEGTACO_TRY(segtaco_spmv_workspace_size(M, nnz, &need));
+    Scratch scratch(workspace, workspace_bytes, s);
+    SEGTACO_TRY(scratch.reserve(need));
   }
-  return run_spmm_planned(plan, M, K, nnz, row_ptr, col, vals, x, SEGTACO_F32, 1, y, 1, 1, px, py,
-                          s);
+  return launch_spmv(M, nnz, row_ptr, col, vals, x, y, s);
 }
 
 int segtaco_sddmm_autotune(int32_t M, int32_t K, int64_t nnz, int32_t D, int32_t x_dtype,

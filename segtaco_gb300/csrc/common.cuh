@@ -417,6 +417,24 @@ __device__ __forceinline__ int merge_path_x(const int *__restrict__ row_ptr, int
   return (int)lo;
 }
 
+// Last row r with row_ptr[r] <= p (the row of nonzero p), found by the whole warp:
+// 32 probes a round.  The first rounds' probes are the same for every warp and
+// stay in L1.
+__device__ __forceinline__ int warp_row_of(const int *__restrict__ row_ptr, int M, long long p,
+                                           int lane) {
+  long long lo = 0, hi = M;  // row_ptr[lo] <= p < row_ptr[hi]
+  while (hi - lo > 1) {
+    const long long step = (hi - lo + 31) / 32;
+    const long long at = lo + (lane + 1) * step;
+    const bool past = at >= hi || (long long)__ldg(row_ptr + at) > p;
+    const int f = __ffs(__ballot_sync(0xffffffffu, past)) - 1;  // lane 31's probe is past hi
+    const long long nhi = lo + (f + 1) * step;
+    lo += f * step;
+    hi = nhi < hi ? nhi : hi;
+  }
+  return (int)lo;
+}
+
 // Merge-path edges by rows instead of by search.  Row end r is merge item
 // e_r - 1 with e_r = row_ptr[r+1] + r + 1, so the split of diagonal d takes
 // x(d) = #{r : e_r <= d} row ends -- exactly the row merge_path_x finds.

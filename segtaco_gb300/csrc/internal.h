@@ -302,6 +302,8 @@ int launch_long_pieces_list(const int *row_ptr, int M, long long nnz, int long_r
 // Multiprocessors of the current device (cached per device).
 int device_sms();
 
+int launch_spmv(int M, long long nnz, const int *row_ptr, const int *col, const float *val,
+                const float *x, float *y, cudaStream_t s);
 int launch_spmspv(int M, int K, const int *col_ptr, const int *row_idx, const float *val, int nx,
                   const int *x_idx, const float *x_vals, float *y, cudaStream_t s);
 
