@@ -65,11 +65,10 @@ extern "C" {
                                      them into registers */
 #define SEGTACO_FLAG_TMA_BULK 8u  /* with SMEM_RING: fill the ring with cp.async.bulk
                                      (TMA) copies rather than 16-byte cp.async copies */
-#define SEGTACO_FLAG_ROW_WALK 16u /* walk each unit row by row (the default except
-                                     for eb_sr; depth 4 or 8 loads in flight)    */
+#define SEGTACO_FLAG_ROW_WALK 16u /* walk each unit row by row (depth 4 or 8 loads
+                                     in flight)                                  */
 #define SEGTACO_FLAG_FLAT_WALK 32u /* walk each unit in batches of 32 nonzeros
-                                      across rows (the default for eb_sr with
-                                      16-byte vectors)                           */
+                                      across rows                                */
 #define SEGTACO_FLAG_LONG_ROWS 64u /* rb schedules with nnz >= 1M: rows of at
                                       least items_per_unit nonzeros are taken
                                       out of the row blocks (see
@@ -135,7 +134,9 @@ typedef struct segtaco_config {
                              piece of a row sums them in piece order, so the
                              result does not vary from run to run          */
   uint32_t flags;         /* SEGTACO_FLAG_*                                        */
-  int32_t depth;          /* row walk: dense loads in flight per lane (0 = 4, 4, 8) */
+  int32_t depth;          /* row walk: dense loads in flight per lane (0 = 4, 4, 8);  */
+                          /* 4 with a row-block schedule: rows are even, several of  */
+                          /* a block are walked side by side                         */
   int32_t k_parts;        /* rb_pr pieces: passes over ranges of B's rows, 1 .. 8
                              (0: one).  With more than one the pieces (of
                              2048 nonzeros) run in a launch of their own

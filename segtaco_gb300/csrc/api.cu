@@ -355,6 +355,35 @@ int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, lo
         (size_t)wrows * W * esz <= 60 * 1024 && window_variant_exists(b_dtype, V, G))
       plan->window_halo = (int)H;
   }
+  // Row blocks of rows known to be even (depth 4, which segtaco_autotune_heuristic sets
+  // for them) without pieces, band or window take the row-slot walk (spmm_rows.cuh)
+  // where a warp holds at least two rows side by side, or the operands allow only 1- or
+  // 2-element lanes.  Measured on GB300, fp32, row walk / row-slot walk: 16,384 rows of
+  // 16, N = 32, rb_sr 9.4 / 4.3 us, rb_pr 8.6 / 4.5; 300,000, N = 16 rb_sr 117 / 30; N = 64
+  // 150 / 97; 20,000 banded rows, N = 37 47 / 26.  Uneven rows keep the row walk: a
+  // slot's trips through a long row cost more instructions than a whole warp's (20,000
+  // power-law rows, N = 37, rb_sr 309 / 937 us).  rb_pr's row walk also splits rows of
+  // more than 32 nonzeros over its slots (50,000 banded rows of 73, N = 32: 29.8 us against
+  // 31.1, N = 16 bf16 23.3 / 27.8; rb_sr 56 / 31).
+  if ((schedule == SEGTACO_RB_SR || schedule == SEGTACO_RB_PR) && c.depth == 4 &&
+      !plan->use_tma && plan->piece_len == 0 && plan->band_halo < 0 && plan->window_halo < 0 &&
+      !(c.flags & (SEGTACO_FLAG_ROW_WALK | SEGTACO_FLAG_FLAT_WALK)) &&
+      ldb * esz < (1LL << 32) && ldc * 4 < (1LL << 32)) {
+    segtaco_config rc = c;
+    if (rc.vec >= 16 / esz) rc.vec = 0;  // (wider lanes: the 16-byte ones)
+    SpmmPlan t = *plan;
+    if (split_shape(rc, N, K, esz, fits, &t) &&
+        (t.split_elems <= 2 ||
+         (t.G < 32 && (schedule == SEGTACO_RB_SR || nnz <= 32LL * M)))) {
+      *plan = t;
+      plan->walk = 6;
+      const int P = 32 / t.G;
+      int rows = P;  // up to four rows per slot, while the warps fill two waves
+      while (2 * rows <= 32 && rows < 4 * P && M / (2 * rows) >= 2 * 152 * 32) rows *= 2;
+      plan->rows_per_unit = rows;
+      plan->nchunks = (M + rows - 1) / rows;
+    }
+  }
   if (plan->px_entries)
     plan->workspace = align256((size_t)plan->px_entries * sizeof(int)) +
                       align256((size_t)plan->py_entries * sizeof(int));
@@ -391,6 +420,8 @@ int run_spmm_planned(const SpmmPlan &plan, int M, int K, long long nnz, const in
   L.deep = plan.deep;
   L.walk = plan.walk;
   L.no_fork = plan.no_fork;
+  L.split_elems = plan.split_elems;
+  L.coop = plan.schedule == SEGTACO_RB_PR;
   L.window_halo = plan.window_halo;
   L.band_halo = plan.band_halo;
   const bool bf16 = b_dtype == SEGTACO_BF16;
@@ -445,7 +476,6 @@ int run_spmm_planned(const SpmmPlan &plan, int M, int K, long long nnz, const in
                                       C, ldc, N, s));
       if (L.use_tma) return bf16 ? launch_spmm_tma_bf16(L, false, s) : launch_spmm_tma_f32(L, false, s);
       if (plan.walk == 5) {
-        L.split_elems = plan.split_elems;
         L.split_items = (int)plan.items_per_unit;
         return bf16 ? launch_spmm_split_bf16(L, s) : launch_spmm_split_f32(L, s);
       }
@@ -569,7 +599,8 @@ int segtaco_autotune_heuristic(int32_t M, int32_t K, int64_t nnz, int32_t N, int
   // nonzeros per row, N = 32: 0.0174 ms with 4 rows, 0.0154 with 2.
   if (schedule == SEGTACO_RB_SR)
     while (cfg->rows_per_unit > 1 && M / cfg->rows_per_unit < 8192) cfg->rows_per_unit >>= 1;
-  cfg->depth = (schedule == SEGTACO_RB_SR || schedule == SEGTACO_RB_PR) ? 8 : 4;
+  // rb: 8 loads in flight in the row walk, or (4) even rows side by side.
+  cfg->depth = (schedule == SEGTACO_RB_SR || schedule == SEGTACO_RB_PR) && !even ? 8 : 4;
   cfg->flags = long_rows ? SEGTACO_FLAG_LONG_ROWS : 0;
   // rb_pr's long rows as pieces of the row-block launch (rows of >= 512
   // nonzeros, pieces of 4096); the rows left are short, so a warp takes 64 of

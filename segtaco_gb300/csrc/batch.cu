@@ -418,16 +418,26 @@ int plan_batch_problem(const segtaco_spmm_problem &p, const segtaco_config *cfg,
   c.flags &= ~(SEGTACO_FLAG_SMEM_RING | SEGTACO_FLAG_TMA_BULK | SEGTACO_FLAG_PARTITION_READY);
   // The persistent kernel walks every row of its items (no long-row CTAs).
   c.flags &= ~SEGTACO_FLAG_LONG_ROWS;
-  SEGTACO_TRY(plan_spmm(p.M, p.K, p.nnz, p.N, p.b_dtype, p.ldb, p.ldc, p.B, p.C, &c, plan));
+  segtaco_config planned = c;  // row blocks: the row walk
+  if ((c.schedule == SEGTACO_RB_SR || c.schedule == SEGTACO_RB_PR) &&
+      !(c.flags & SEGTACO_FLAG_FLAT_WALK))
+    planned.flags |= SEGTACO_FLAG_ROW_WALK;
+  SEGTACO_TRY(
+      plan_spmm(p.M, p.K, p.nnz, p.N, p.b_dtype, p.ldb, p.ldc, p.B, p.C, &planned, plan));
   // The persistent kernel hides the row walk's round trips behind other problems'
   // items, so the split walk pays there where it saves passes over A or narrow
   // loads: slabs of more than 64 columns, and operands without 16-byte lanes, over
   // chunks of 128 items.  Measured on GB300, the pool's problems of one N, row walk
   // (slabs of up to 64 columns) / split walk at 128 and 256 items: N = 16 152 / 213
-  // / 187 us, 32 105 / 120 / 112, 64 131 / 131 / 129, 128 117 / 86 / 105.
+  // / 187 us, 32 105 / 120 / 112, 64 131 / 131 / 129, 128 117 / 86 / 105.  A product of
+  // fewer than 300,000 items keeps the row walk whatever its slab: batches whose wide
+  // products are all that small end on a nearly empty split group (16 problems, three
+  // wide ones of up to 257,000 items: 136 us against 146), and beside larger ones they
+  // cost the same either way (24 problems 434 / 450, 48 problems 395 / 395).
   if (plan->walk == kWalkSplit && !cfg) {
     const int esz = p.b_dtype == SEGTACO_BF16 ? 2 : 4;
-    if (plan->split_elems * esz == 16 && plan->W <= 64) {
+    if (plan->split_elems * esz == 16 &&
+        (plan->W <= 64 || (long long)p.M + p.nnz < 300000)) {
       if (c.col_tile <= 0) c.col_tile = std::min(p.N, 256 / esz);
       segtaco_config rows = c;
       rows.flags |= SEGTACO_FLAG_ROW_WALK;

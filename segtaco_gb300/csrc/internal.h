@@ -82,6 +82,7 @@ struct SpmmLaunch {
   int carveout = -1;           // >= 0: preferred shared-memory carveout (%) of the launch
   int split_elems = 0;         // split walk: elements per lane chunk (V / split_elems chunks)
   int split_items = 0;         // split walk: merge-path items per chunk
+  bool coop = false;           // rb_pr: longer rows by a whole warp or CTA, any order
   bool no_fork = false;        // rb long rows: both kernels on the call's stream (no side
                                // stream or events are created)
   int window_halo = -1;        // >= 0: rb rows with B rows [i0 - halo, i1 + halo) of each
@@ -110,6 +111,9 @@ int launch_spmm_bf16_chunks(const SpmmLaunch &L, cudaStream_t s);
 // The split walk of merge-path chunks (spmm_split.cuh).
 int launch_spmm_split_f32(const SpmmLaunch &L, cudaStream_t s);
 int launch_spmm_split_bf16(const SpmmLaunch &L, cudaStream_t s);
+// The row-slot walk of row blocks (spmm_rows.cuh).
+int launch_spmm_slots_f32(const SpmmLaunch &L, cudaStream_t s);
+int launch_spmm_slots_bf16(const SpmmLaunch &L, cudaStream_t s);
 // rb_pr's pieces in piece_parts passes (a persistent launch before the row
 // blocks).
 int launch_spmm_pieces_f32(const SpmmLaunch &L, cudaStream_t s);
@@ -139,7 +143,7 @@ struct SpmmPlan {
   bool bulk_copies;
   bool deep;
   int walk;                  // kWalkRows / kWalkRowsDeep / kWalkFlat / ... / kWalkSplit
-  int split_elems = 0;       // split walk: elements per lane chunk
+  int split_elems = 0;       // split and row-slot walks: elements per lane chunk
   int long_row;              // rb: long-row threshold (0: every row in the row-block kernel)
   bool no_fork = false;      // rb long rows: no side stream (segtaco_spmm_noalloc)
   int window_halo = -1;      // rb: >= 0 stages each row block's B window (spmm_window.cu)

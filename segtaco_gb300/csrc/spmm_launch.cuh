@@ -147,6 +147,8 @@ inline dim3 spmm_grid(const SpmmLaunch &L) {
 #define SEGTACO_DEFINE_SPMM_LAUNCHER(NAME, BT, VG_LIST, ROWS)                             \
   namespace segtaco {                                                                     \
   int NAME(const SpmmLaunch &L, cudaStream_t s) {                                         \
+    if (ROWS && L.walk == kWalkRowSlots)                                                  \
+      return sizeof(BT) == 4 ? launch_spmm_slots_f32(L, s) : launch_spmm_slots_bf16(L, s); \
     const SpmmArgs<BT> a = make_spmm_args<BT>(L);                                         \
     const dim3 grid = spmm_grid(L);                                                       \
     if constexpr (!ROWS) {                                                                \

@@ -355,8 +355,7 @@ int launch_long_typed(const SpmmLaunch &L, const int *list, int *counters, int s
                       cudaStream_t s) {
   const SpmmArgs<BT> a = make_spmm_args<BT>(L);
   // Slabs of 128 columns (one per row at N <= 128); 32 or 64 for narrower N.
-  // rb_sr plans one slot of 32 lanes (G = 32), rb_pr several.
-  if (L.G == 32) {
+  if (!L.coop) {  // rb_sr
     // The row-block kernel's slab width (its B working set) where narrower.
     const int W = L.V * L.G;
     if (L.N <= 32 || W <= 32) return launch_long_kernel<BT, 32, false>(a, list, counters, sms, s);
