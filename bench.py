@@ -1040,6 +1040,8 @@ def launches_per_step(eb, ws_need, plan):
         return 2
     if " pieces " in plan:
         return 3 if not plan.endswith(" parts=1") else 2
+    if " walk=7 " in plan:  # rb_pr's joined chunks: product + sums of cut rows
+        return 2
     return 3 if ws_need else 1
 
 

@@ -136,7 +136,11 @@ typedef struct segtaco_config {
   uint32_t flags;         /* SEGTACO_FLAG_*                                        */
   int32_t depth;          /* row walk: dense loads in flight per lane (0 = 4, 4, 8);  */
                           /* 4 with a row-block schedule: rows are even, several of  */
-                          /* a block are walked side by side                         */
+                          /* a block are walked side by side; 8 with rb_pr and       */
+                          /* SEGTACO_FLAG_LONG_ROWS: rows are uneven, equal chunks   */
+                          /* of the matrix are walked and the rows they cut summed   */
+                          /* in order (any nnz; not with fp32 vec 8 or k_parts > 1;  */
+                          /* where the workspace holds the sums)                     */
   int32_t k_parts;        /* rb_pr pieces: passes over ranges of B's rows, 1 .. 8
                              (0: one).  With more than one the pieces (of
                              2048 nonzeros) run in a launch of their own

@@ -1,5 +1,6 @@
 // api.cu -- the extern "C" entry points of include/segtaco.h, argument checks,
 // scratch handling and the SpMM planner (schedule / slab width / vector width).
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -174,7 +175,7 @@ static bool split_shape(const segtaco_config &c, int N, int K, int esz, F fits, 
 
 int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, long long ldc,
               const void *B, const float *C, const segtaco_config *cfg, SpmmPlan *plan,
-              bool pieces) {
+              LongRowScratch scratch) {
   segtaco_config c{};
   c.schedule = SEGTACO_AUTO;
   if (cfg) c = *cfg;
@@ -298,7 +299,7 @@ int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, lo
   } else if (nnz >= kLongRowsMinNnz && (c.flags & SEGTACO_FLAG_LONG_ROWS) &&
              plan->walk != 2 && !plan->use_tma) {
     const int epc = 16 / esz;
-    if (schedule == SEGTACO_RB_PR && pieces) {
+    if (schedule == SEGTACO_RB_PR && scratch != LongRowScratch::kList) {
       // rb_pr: long rows as pieces of kPieceLen nonzeros in the row-block
       // launch (spmm_long.cu), over the same column slabs; rows from
       // kPieceThreshold nonzeros by default.
@@ -332,7 +333,7 @@ int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, lo
       !(c.flags & (SEGTACO_FLAG_ROW_WALK | SEGTACO_FLAG_FLAT_WALK)) && c.depth != 8 &&
       ldb * esz < (1LL << 32) && ldc * 4 < (1LL << 32) &&
       split_shape(c, N, K, esz, fits, plan))
-    plan->walk = 5;
+    plan->walk = kWalkSplit;
   plan->window_halo = -1;
   plan->band_halo = -1;
   if ((c.flags & SEGTACO_FLAG_WINDOW) && schedule == SEGTACO_RB_PR && plan->long_row == 0 &&
@@ -376,12 +377,31 @@ int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, lo
         (t.split_elems <= 2 ||
          (t.G < 32 && (schedule == SEGTACO_RB_SR || nnz <= 32LL * M)))) {
       *plan = t;
-      plan->walk = 6;
+      plan->walk = kWalkRowSlots;
       const int P = 32 / t.G;
       int rows = P;  // up to four rows per slot, while the warps fill two waves
       while (2 * rows <= 32 && rows < 4 * P && M / (2 * rows) >= 2 * 152 * 32) rows *= 2;
       plan->rows_per_unit = rows;
       plan->nchunks = (M + rows - 1) / rows;
+    }
+  }
+  // rb_pr over rows known to be uneven (depth 8 with SEGTACO_FLAG_LONG_ROWS, which
+  // segtaco_autotune_heuristic sets for them): merge-path chunks whose sums of cut
+  // rows are added in order (spmm_join.cu) instead of pieces and row blocks.  fp32's
+  // explicit 32-byte lanes (split_shape) and passes over B keep the pieces.
+  if (schedule == SEGTACO_RB_PR && scratch == LongRowScratch::kJoin && nnz > 0 && c.depth == 8 &&
+      c.k_parts <= 1 && (c.flags & SEGTACO_FLAG_LONG_ROWS) && !plan->use_tma &&
+      plan->band_halo < 0 && plan->window_halo < 0 &&
+      !(c.flags & (SEGTACO_FLAG_ROW_WALK | SEGTACO_FLAG_FLAT_WALK)) &&
+      ldb * esz < (1LL << 32) && ldc * 4 < (1LL << 32)) {
+    if (split_shape(c, N, K, esz, fits, plan)) {
+      plan->walk = kWalkSplitJoin;
+      plan->long_row = plan->piece_len = 0;
+      plan->piece_parts = 1;
+      plan->items_per_unit = default_chunk_items(M, nnz);
+      plan->nchunks = (M + nnz + plan->items_per_unit - 1) / plan->items_per_unit;
+      plan->px_entries = 2 * plan->nchunks * (((long long)N + 3) & ~3LL);
+      plan->py_entries = 0;
     }
   }
   if (plan->px_entries)
@@ -431,6 +451,14 @@ int run_spmm_planned(const SpmmPlan &plan, int M, int K, long long nnz, const in
       if (L.use_tma) return bf16 ? launch_spmm_tma_bf16(L, true, s) : launch_spmm_tma_f32(L, true, s);
       if (plan.band_halo >= 0) return launch_spmm_band(L, s);
       if (plan.window_halo >= 0) return launch_spmm_window(L, s);
+      if (plan.walk == kWalkSplitJoin) {
+        L.part_x = L.part_y = nullptr;  // the edges are searched in the kernels
+        L.split_items = (int)plan.items_per_unit;
+        L.piece_part = reinterpret_cast<float *>(px);
+        L.piece_ld = ((long long)N + 3) & ~3LL;
+        SEGTACO_TRY(bf16 ? launch_spmm_join_bf16(L, s) : launch_spmm_join_f32(L, s));
+        return launch_spmm_join(L, s);
+      }
       if (plan.long_row > 0 && plan.piece_len > 0) {
         L.long_row = plan.long_row;
         if (!partition_ready)
@@ -475,7 +503,7 @@ int run_spmm_planned(const SpmmPlan &plan, int M, int K, long long nnz, const in
         SEGTACO_TRY(launch_merge_path(row_ptr, M, nnz, plan.items_per_unit, plan.nchunks, px, py,
                                       C, ldc, N, s));
       if (L.use_tma) return bf16 ? launch_spmm_tma_bf16(L, false, s) : launch_spmm_tma_f32(L, false, s);
-      if (plan.walk == 5) {
+      if (plan.walk == kWalkSplit) {
         L.split_items = (int)plan.items_per_unit;
         return bf16 ? launch_spmm_split_bf16(L, s) : launch_spmm_split_f32(L, s);
       }
@@ -576,6 +604,16 @@ int segtaco_autotune_heuristic(int32_t M, int32_t K, int64_t nnz, int32_t N, int
   // N = 64) 120 / 105.
   const bool heavy = (double)max_row_len > 256.0 * mean && bbytes > 96e6;
   const bool split = schedule == SEGTACO_EB_PR && !(heavy && N % (32 / esz) == 0);
+  // rb_pr takes chunks whose cut rows are joined (spmm_join.cu) from the same longest
+  // rows as the pieces, and below 1M nonzeros from 640, with the same exception for
+  // fp32.  Measured on GB300, row walk / joined chunks (longest row): 1000 power-law
+  // rows, N = 16 8.2 / 9.3 us (513), 1473, N = 114 26.0 / 11.7 (1267), 17,801, N = 97 679 / 38
+  // (26,528); lognormal rows, N = 64, 3000 8.6 / 10.9 (209), 80,000 39.6 / 31.4 (796).
+  // Pieces / joined chunks, power-law rows: 60,000, N = 64 108 / 45, 400,000, N = 37 432 /
+  // 183, N = 128 372 / 420 fp32 and 301 / 274 bf16; 400,000 lognormal rows, N = 128 395 / 278.
+  const bool join = schedule == SEGTACO_RB_PR && !even && !(heavy && esz == 4 && N % 8 == 0) &&
+                    (long_rows || (nnz < kLongRowsMinNnz && max_row_len >= 640 &&
+                                   !(banded && N >= 64 && N % 16 == 0)));
   // A B that fits L2 whole (up to ~96 MB) under a large product: one slab of
   // up to 64 columns (8 per lane, G = 8), so A is read once.  Measured on
   // GB300, banded 262,144 rows (19.1M nonzeros), N = 64, rb_pr: 0.248 ms
@@ -583,12 +621,12 @@ int segtaco_autotune_heuristic(int32_t M, int32_t K, int64_t nnz, int32_t N, int
   if (!sequential && esz == 4 && bbytes > 48e6 && bbytes <= 96e6 && nnz >= 4000000 &&
       N % 8 == 0 && !skewed)
     cfg->col_tile = N < 64 ? N : 64;
-  if (split) cfg->col_tile = cfg->vec = 0;
   // bf16 likewise: 16 columns per lane (one 32-byte load) on 64-column slabs.
   // Measured on GB300: 1M x 1M power law, N = 128, eb_pr 0.996 -> 0.823 ms;
   // with B in L2 (banded, N = 64) 8 stays faster (0.224 vs 0.235 ms).
   if (!sequential && esz == 2 && bbytes > 48e6 && N % 16 == 0 && (skewed || nnz >= 4000000))
     cfg->vec = 16;
+  if (split || join) cfg->col_tile = cfg->vec = 0;
   // eb: merge-path items per chunk; rb: the long-row threshold.
   cfg->items_per_unit = (schedule == SEGTACO_RB_SR || schedule == SEGTACO_RB_PR)
                             ? (int)kLongRowDefault
@@ -601,7 +639,7 @@ int segtaco_autotune_heuristic(int32_t M, int32_t K, int64_t nnz, int32_t N, int
     while (cfg->rows_per_unit > 1 && M / cfg->rows_per_unit < 8192) cfg->rows_per_unit >>= 1;
   // rb: 8 loads in flight in the row walk, or (4) even rows side by side.
   cfg->depth = (schedule == SEGTACO_RB_SR || schedule == SEGTACO_RB_PR) && !even ? 8 : 4;
-  cfg->flags = long_rows ? SEGTACO_FLAG_LONG_ROWS : 0;
+  cfg->flags = long_rows || join ? SEGTACO_FLAG_LONG_ROWS : 0;
   // rb_pr's long rows as pieces of the row-block launch (rows of >= 512
   // nonzeros, pieces of 4096); the rows left are short, so a warp takes 64 of
   // them to fill its slots (32 while that leaves fewer than 8192 warps).
@@ -664,6 +702,11 @@ int segtaco_spmm_workspace_size(int32_t M, int32_t K, int64_t nnz, int32_t N, in
   // Alignment does not change the workspace: plan with aligned stand-ins.
   SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, N, N, nullptr, nullptr, cfg, &plan));
   *bytes = plan.workspace;
+  if (plan.walk == kWalkSplitJoin) {  // (row pitches from 4 GB keep the pieces)
+    SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, N, N, nullptr, nullptr, cfg, &plan,
+                          LongRowScratch::kPieces));
+    *bytes = std::max(*bytes, plan.workspace);
+  }
   return SEGTACO_OK;
 }
 
@@ -681,9 +724,13 @@ int segtaco_spmm(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr, cons
   if (ldb < N || ldc < N) return set_error(SEGTACO_EINVAL, "ldb/ldc smaller than N");
   SpmmPlan plan;
   SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, ldb, ldc, B, C, cfg, &plan));
+  // A caller's workspace without room for the sums of cut rows: the pieces or row blocks
+  if (plan.walk == kWalkSplitJoin && workspace && workspace_bytes < plan.workspace)
+    SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, ldb, ldc, B, C, cfg, &plan,
+                          LongRowScratch::kPieces));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool ready = cfg && (cfg->flags & SEGTACO_FLAG_PARTITION_READY);
-  const bool search = !ready && plan.walk == 5 && (long long)M * N <= kSearchMaxElems;
+  const bool search = !ready && plan.walk == kWalkSplit && (long long)M * N <= kSearchMaxElems;
   Scratch scratch(workspace, workspace_bytes, s);
   if (workspace || !search)  // (a caller's workspace is checked, if not needed)
     SEGTACO_TRY(scratch.reserve(plan.workspace));
@@ -692,7 +739,7 @@ int segtaco_spmm(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr, cons
     px = static_cast<int *>(scratch.take(plan.px_entries * sizeof(int)));
     py = static_cast<int *>(scratch.take(plan.py_entries * sizeof(int)));
   }
-  if (ready && plan.workspace && !workspace)
+  if (ready && plan.workspace && !workspace && plan.walk != kWalkSplitJoin)
     return set_error(SEGTACO_EINVAL, "PARTITION_READY needs the caller's workspace");
   return run_spmm_planned(plan, M, K, nnz, row_ptr, col, vals, B, b_dtype, ldb, C, ldc, N, px, py,
                           s, ready);
@@ -706,6 +753,11 @@ int segtaco_spmm_partition(int32_t M, int32_t K, int64_t nnz, const int32_t *row
   if (C == nullptr || ldc < N) return set_error(SEGTACO_EINVAL, "C is NULL or ldc < N");
   SpmmPlan plan;
   SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, N, ldc, nullptr, C, cfg, &plan));
+  if (plan.walk == kWalkSplitJoin && workspace_bytes >= plan.workspace)
+    return SEGTACO_OK;  // nothing to prepare
+  if (plan.walk == kWalkSplitJoin)
+    SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, N, ldc, nullptr, C, cfg, &plan,
+                          LongRowScratch::kPieces));
   if (!plan.workspace) return SEGTACO_OK;
   if (!workspace) return set_error(SEGTACO_EINVAL, "segtaco_spmm_partition needs a workspace");
   cudaStream_t s = static_cast<cudaStream_t>(stream);

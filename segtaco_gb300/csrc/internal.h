@@ -58,6 +58,10 @@ int launch_row_ids(const int *row_ptr, int M, int *out, cudaStream_t s);
 int launch_validate(const int *row_ptr, int M, int K, long long nnz, const int *col, int *err,
                     cudaStream_t s);
 
+// Walks beside those of spmm_kernels.cuh: merge-path chunks (spmm_split.cuh), row slots
+// (spmm_rows.cuh), merge-path chunks joined in order (spmm_join.cu).
+constexpr int kWalkSplit = 5, kWalkRowSlots = 6, kWalkSplitJoin = 7;
+
 // ---- SpMM kernel launch description (spmm_*.cu) ----
 struct SpmmLaunch {
   int dtype;     // SEGTACO_F32 / SEGTACO_BF16
@@ -77,7 +81,7 @@ struct SpmmLaunch {
   bool use_tma;                // gather B into a shared-memory ring (spmm_tma.cuh)
   bool bulk_copies;            // ... with cp.async.bulk (TMA) rather than cp.async
   bool deep;                   // row walk: 8 sixteen-byte loads in flight per lane
-  int walk;                    // kWalkRows / kWalkRowsDeep / kWalkFlat (spmm_kernels.cuh)
+  int walk;                    // kWalk...
   int long_row = 0;            // rb: rows of >= long_row nonzeros go to spmm_long.cu
   int carveout = -1;           // >= 0: preferred shared-memory carveout (%) of the launch
   int split_elems = 0;         // split walk: elements per lane chunk (V / split_elems chunks)
@@ -111,6 +115,10 @@ int launch_spmm_bf16_chunks(const SpmmLaunch &L, cudaStream_t s);
 // The split walk of merge-path chunks (spmm_split.cuh).
 int launch_spmm_split_f32(const SpmmLaunch &L, cudaStream_t s);
 int launch_spmm_split_bf16(const SpmmLaunch &L, cudaStream_t s);
+// The same with the sums of cut rows left in L.piece_part, and their addition (spmm_join.cu).
+int launch_spmm_join_f32(const SpmmLaunch &L, cudaStream_t s);
+int launch_spmm_join_bf16(const SpmmLaunch &L, cudaStream_t s);
+int launch_spmm_join(const SpmmLaunch &L, cudaStream_t s);
 // The row-slot walk of row blocks (spmm_rows.cuh).
 int launch_spmm_slots_f32(const SpmmLaunch &L, cudaStream_t s);
 int launch_spmm_slots_bf16(const SpmmLaunch &L, cudaStream_t s);
@@ -142,7 +150,7 @@ struct SpmmPlan {
   bool use_tma;
   bool bulk_copies;
   bool deep;
-  int walk;                  // kWalkRows / kWalkRowsDeep / kWalkFlat / ... / kWalkSplit
+  int walk;                  // kWalk...
   int split_elems = 0;       // split and row-slot walks: elements per lane chunk
   int long_row;              // rb: long-row threshold (0: every row in the row-block kernel)
   bool no_fork = false;      // rb long rows: no side stream (segtaco_spmm_noalloc)
@@ -156,10 +164,12 @@ struct SpmmPlan {
   long long py_entries;      // ... of the second (eb: chunk-edge nonzeros; long rows: counters)
   size_t workspace;          // bytes
 };
-// `pieces` false: rb_pr long rows go to the long-row CTAs, as for rb_sr.
+// What the workspace has room for under rb_pr's long rows: the sums of joined chunks
+// (spmm_join.cu), else pieces, else the list of the long-row CTAs, as for rb_sr.
+enum class LongRowScratch { kList, kPieces, kJoin };
 int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, long long ldc,
               const void *B, const float *C, const segtaco_config *cfg, SpmmPlan *plan,
-              bool pieces = true);
+              LongRowScratch scratch = LongRowScratch::kJoin);
 // Runs a planned SpMM with partition arrays already in `px/py` (eb) or none.
 int run_spmm_planned(const SpmmPlan &plan, int M, int K, long long nnz, const int *row_ptr,
                      const int *col, const float *vals, const void *B, int b_dtype, long long ldb,

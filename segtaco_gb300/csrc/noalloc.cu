@@ -80,10 +80,13 @@ extern "C" int segtaco_spmm_noalloc(int32_t M, int32_t K, int64_t nnz, const int
     return set_error(SEGTACO_EINVAL,
                      "segtaco_spmm_noalloc: PARTITION_READY is not supported (shared scratch)");
   SpmmPlan plan;
-  SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, ldb, ldc, B, C, cfg, &plan));
+  // (no joined chunks: below 1M nonzeros rb_pr keeps off the shared scratch)
+  SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, ldb, ldc, B, C, cfg, &plan,
+                        LongRowScratch::kPieces));
   if (plan.piece_len > 0 && plan.px_entries > kNoallocEntries)
     // rb_pr pieces whose partial rows would not fit: the long-row CTAs
-    SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, ldb, ldc, B, C, cfg, &plan, false));
+    SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, ldb, ldc, B, C, cfg, &plan,
+                          LongRowScratch::kList));
   plan.no_fork = true;  // rb long rows: no side stream or events, both kernels on `stream`
   if (plan.long_row > 0 && plan.px_entries > kNoallocEntries) {
     // the long-row list would not fit: every row in the row-block kernel

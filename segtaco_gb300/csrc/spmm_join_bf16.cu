@@ -1,0 +1,5 @@
+// Split walk of merge-path chunks whose cut rows are joined, bf16 dense operand (bit patterns as
+// uint16_t).
+#include "spmm_split_launch.cuh"
+
+SEGTACO_DEFINE_SPLIT_LAUNCHER(launch_spmm_join_bf16, uint16_t, SEGTACO_SPLIT_BF16, SEGTACO_JOIN_CASE)

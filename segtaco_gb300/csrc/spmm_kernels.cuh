@@ -966,8 +966,6 @@ __device__ __forceinline__ void spmm_seq_unit(const SpmmArgs<BT> &a, long long w
 // flat walk, the slot walk or the sequential walk over merge-path chunks
 // (chosen by the planner, api.cu).
 constexpr int kWalkRows = 0, kWalkRowsDeep = 1, kWalkFlat = 2, kWalkSlots = 3, kWalkSeq = 4;
-constexpr int kWalkSplit = 5;    // spmm_split.cuh
-constexpr int kWalkRowSlots = 6;  // spmm_rows.cuh
 
 // CTAs of the SpMM kernels: 4 warps each, so a CTA that finishes early frees
 // its slot soon (warps of a CTA walk units of uneven cost).  32 warps per SM

@@ -100,10 +100,13 @@ __device__ __forceinline__ ChunkEdges search_edges(const SpmmArgs<BT> &a, long l
           __shfl_sync(FULL, y, 16)};
 }
 
-template <typename BT, int E, int C, int G>
+// JOIN (rb_pr, spmm_join.cu): chunk w's sums of rows cut by its edges are stored in
+// a.piece_part -- two rows of a.piece_ld floats, the row it starts in, then the row
+// open at its end -- instead of being added to C.
+template <typename BT, int E, int C, int G, bool JOIN = false>
 __device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, const ChunkEdges ce,
                                                 int slab, int lane, int D,
-                                                int *__restrict__ sm) {
+                                                int *__restrict__ sm, long long w = 0) {
   constexpr int P = 32 / G;
   constexpr int V = E * C;
   constexpr int S = kSplitStep;
@@ -285,13 +288,14 @@ __device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, const Chu
 #pragma unroll
     for (int v = 0; v < V; ++v) acc[v] = head[v];
     add_open(slot - 1);
-    store(c_row(x0 + hrow), hrow == 0 && head_split);
+    const bool cut = hrow == 0 && head_split;
+    store(JOIN && cut ? a.piece_part + 2 * w * a.piece_ld + col0 : c_row(x0 + hrow), !JOIN && cut);
   }
   // The row open at the chunk's end (it ends in a later chunk).
   if (slot == 0 && x1 < M && __ldg(a.row_ptr + x1) < y1) {
     zero<V>(acc);
     add_open(P - 1);
-    store(c_row(x1), true);
+    store(JOIN ? a.piece_part + (2 * w + 1) * a.piece_ld + col0 : c_row(x1), !JOIN);
   }
 }
 
@@ -299,8 +303,9 @@ template <typename BT, int E, int C, int G> constexpr int split_min_ctas() {
   return (E * C * sizeof(BT) > 16 || C > 1 ? 32 : 36) / kSpmmWarps;
 }
 
-// a.part_x null: the chunk's edges are searched here and C is zero on entry.
-template <typename BT, int E, int C, int G>
+// a.part_x null: the chunk's edges are searched here (and, but for JOIN, C is zero on
+// entry).
+template <typename BT, int E, int C, int G, bool JOIN = false>
 __global__ void __launch_bounds__(kSpmmCta, split_min_ctas<BT, E, C, G>())
     spmm_split_kernel(SpmmArgs<BT> a, int D) {
   extern __shared__ __align__(16) int split_sm[];
@@ -308,8 +313,8 @@ __global__ void __launch_bounds__(kSpmmCta, split_min_ctas<BT, E, C, G>())
   if (w >= a.units) return;  // whole warp leaves together
   const int lane = threadIdx.x & 31;
   const ChunkEdges ce = a.part_x ? chunk_edges(a, w) : search_edges(a, w, D, lane);
-  spmm_split_unit<BT, E, C, G>(a, ce, blockIdx.y, lane, D,
-                               split_sm + threadIdx.x / 32 * split_words<E * C>(D));
+  spmm_split_unit<BT, E, C, G, JOIN>(a, ce, blockIdx.y, lane, D,
+                                     split_sm + threadIdx.x / 32 * split_words<E * C>(D), w);
 }
 
 }  // namespace segtaco

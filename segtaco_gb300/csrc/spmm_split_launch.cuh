@@ -22,12 +22,14 @@
   X(uint16_t, 4, 1, 32) SEGTACO_SPLIT_NARROW(X, uint16_t)
 
 #define SEGTACO_SPLIT_KEY(E, C, G) ((E)*10000 + (C)*100 + (G))
-#define SEGTACO_SPLIT_CASE(BT, E, C, G)                                                    \
+#define SEGTACO_SPLIT_RUN(BT, E, C, G, JOIN)                                               \
   case SEGTACO_SPLIT_KEY(E, C, G):                                                         \
-    spmm_split_kernel<BT, E, C, G><<<grid, kSpmmCta, split_bytes<(E) * (C)>(L.split_items), s>>>( \
-        a, L.split_items);                                                                 \
+    spmm_split_kernel<BT, E, C, G, JOIN>                                                   \
+        <<<grid, kSpmmCta, split_bytes<(E) * (C)>(L.split_items), s>>>(a, L.split_items);  \
     break;
-#define SEGTACO_DEFINE_SPLIT_LAUNCHER(NAME, BT, LIST)                                      \
+#define SEGTACO_SPLIT_CASE(BT, E, C, G) SEGTACO_SPLIT_RUN(BT, E, C, G, false)
+#define SEGTACO_JOIN_CASE(BT, E, C, G) SEGTACO_SPLIT_RUN(BT, E, C, G, true)
+#define SEGTACO_DEFINE_SPLIT_LAUNCHER(NAME, BT, LIST, CASE)                                \
   namespace segtaco {                                                                      \
   int NAME(const SpmmLaunch &L, cudaStream_t s) {                                          \
     const SpmmArgs<BT> a = make_spmm_args<BT>(L);                                          \
@@ -36,7 +38,7 @@
                     (unsigned)((L.N + W - 1) / W), 1);                                     \
     const int E = L.split_elems;                                                           \
     switch (SEGTACO_SPLIT_KEY(E, L.V / E, L.G)) {                                          \
-      LIST(SEGTACO_SPLIT_CASE)                                                             \
+      LIST(CASE)                                                                           \
       default:                                                                             \
         return set_error(SEGTACO_EUNSUPPORTED, #NAME ": no variant E=%d V=%d G=%d", E, L.V, L.G); \
     }                                                                                      \
