@@ -663,7 +663,7 @@ int segtaco_autotune_heuristic(int32_t M, int32_t K, int64_t nnz, int32_t N, int
   // rb_pr takes the band kernel (32-row blocks, the band of A as a dense tile,
   // B's window by TMA, 4 x 4 register tiles; spmm_window.cu) with a halo of
   // 32.  Measured on GB300, banded-plus-random 262,144 rows (half band 32, 8
-  // off-band nonzeros per row): fp32 N = 64 0.2465 -> 0.195 ms, bf16 B
+  // off-band nonzeros per row): fp32 N = 64 0.2465 -> 0.181 ms, bf16 B
   // 0.2323 -> 0.114 ms, fp32 N = 128 0.650 -> 0.455 ms (halo 16: 0.61 ms,
   // 48: 0.29 ms at fp32 N = 64).  The staged window for the row-block walk
   // (still one gathered B slice per nonzero, from shared memory instead of

@@ -124,12 +124,13 @@ __global__ void __launch_bounds__(kSpmmCta, window_min_ctas<BT, V, G>())
 // order within a row differs from the storage order, which the parallel
 // reduction allows; duplicate entries of a row add up in the tile.
 //
-// The scatter reads the block's nonzeros (contiguous in A) coalesced, finding
-// each one's row among the 33 staged row starts; off-band nonzeros (outside
-// the window) go to a per-row list of kBandList entries, and each thread
-// gathers its 4 columns of them from global memory, 8 at a time (a row with
-// more walks its nonzeros in global memory instead).  The TMA wait is bounded
-// as in the window kernel (SEGTACO_ETIMEOUT, rows left unwritten).
+// The scatter reads the block's nonzeros (contiguous in A) coalesced, 20 per thread in
+// flight, one exchange per nonzero (with 8, a row search each and float adds in shared
+// memory: banded 262,144 rows, N = 64 195 us, now 181; 100,000, N = 128 144, now 133).
+// Off-band nonzeros (outside the window) go to a per-row list of kBandList entries,
+// and each thread gathers its 4 columns of them from global memory, 8 at a time (a
+// row with more walks its nonzeros in global memory instead).  The TMA wait is
+// bounded as in the window kernel (SEGTACO_ETIMEOUT, rows left unwritten).
 constexpr int kBandRows = 32;
 constexpr int kBandCols = 64;
 constexpr int kBandList = 16;
@@ -188,15 +189,8 @@ __global__ void __launch_bounds__(kSpmmCta)
   if (t == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  for (int e = t; e < win * kBandPitch / 4; e += kSpmmCta)
-    reinterpret_cast<float4 *>(at)[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  if (t <= kBandRows) rp[t] = __ldg(a.row_ptr + min(i0 + t, M));
-  if (t < kBandRows) cnt[t] = 0;
-  __syncthreads();
-  if (t == 0) {
-    const uint32_t bytes = (uint32_t)((size_t)win * kBandCols * sizeof(float));
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes)
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b),
+                 "r"((uint32_t)((size_t)win * kBandCols * sizeof(float)))
                  : "memory");
     // x = the slab's first column (a multiple of 64 elements), y = the
     // window's first row (negative at the top edge: zero-filled)
@@ -206,30 +200,46 @@ __global__ void __launch_bounds__(kSpmmCta)
         "l"(&tm), "r"((int)(blockIdx.y * kBandCols)), "r"(jw0), "r"(b)
         : "memory");
   }
-  // Scatter the block's nonzeros rp[0] .. rp[32]-1, eight per thread per pass
-  // (loads first, then the row searches and shared-memory updates).
-  constexpr int SQ = 8;
-  const int k_end = rp[kBandRows];
-  for (int k0 = rp[0] + t; k0 < k_end; k0 += SQ * kSpmmCta) {
-    int cj[SQ];
-    float cv[SQ];
+  // Scatter the block's nonzeros, SQ per thread per pass with every load in flight;
+  // the first pass loads before the tile is cleared.  An exchange puts a value in
+  // the tile; where it returns another entry of the same position, that one is added
+  // back (the native exchange is one instruction, an add of floats in shared memory a
+  // loop).
+  constexpr int SQ = 20;
+  const int k_beg = __ldg(a.row_ptr + i0), k_end = __ldg(a.row_ptr + min(i0 + kBandRows, M));
+  int cj[SQ];
+  float cv[SQ];
+  auto load = [&](int n0) {  // nonzeros k_beg + n0 + t + 128 q
 #pragma unroll
     for (int q = 0; q < SQ; ++q) {
-      const int k = k0 + q * kSpmmCta;
-      cj[q] = k < k_end ? __ldg(a.col + k) : 0;
-      cv[q] = k < k_end ? ld_val(a.val, k) : 0.0f;
+      const bool has = n0 + t + q * kSpmmCta < k_end - k_beg;
+      cj[q] = has ? __ldg(a.col + (k_beg + n0 + t + q * kSpmmCta)) : 0;
+      cv[q] = has ? ld_val(a.val, k_beg + n0 + t + q * kSpmmCta) : 0.0f;
     }
+  };
+  load(0);
+  for (int e = t; e < win * kBandPitch / 4; e += kSpmmCta)
+    reinterpret_cast<float4 *>(at)[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (t <= kBandRows) rp[t] = __ldg(a.row_ptr + min(i0 + t, M));
+  if (t < kBandRows) cnt[t] = 0;
+  __syncthreads();
+  for (int n0 = 0; n0 < k_end - k_beg; n0 += SQ * kSpmmCta) {
+    if (n0 > 0) load(n0);
+    int r = 0;  // the last row whose start is <= the thread's first nonzero
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (r + step <= kBandRows - 1 && rp[r + step] - k_beg <= n0 + t) r += step;
+    int rend = rp[r + 1] - k_beg;
 #pragma unroll
     for (int q = 0; q < SQ; ++q) {
-      const int k = k0 + q * kSpmmCta;
-      if (k < k_end) {
-        int r = 0;  // the last row whose start is <= k
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1)
-          if (r + step <= kBandRows - 1 && rp[r + step] <= k) r += step;
+      const int n = n0 + t + q * kSpmmCta;
+      if (n < k_end - k_beg) {
+        while (n >= rend) rend = rp[++r + 1] - k_beg;  // n < rp[kBandRows] - k_beg
         const unsigned d = (unsigned)(cj[q] - jw0);
         if (d < (unsigned)win) {
-          atomicAdd(at + d * kBandPitch + r, cv[q]);
+          float *cell = at + d * kBandPitch + r;
+          const float old = atomicExch(cell, cv[q]);
+          if (old != 0.0f) atomicAdd(cell, old);
         } else {
           const int slot = atomicAdd(cnt + r, 1);
           if (slot < kBandList) {
