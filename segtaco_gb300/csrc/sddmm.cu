@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kCta, 3) sddmm_kernel(int M, long long nnz,
 // per multiply-add).  The row of a warp's first nonzero is searched in the kernel,
 // so a call is one launch and needs no scratch.  Measured on GB300, call time, the
 // kernels below (block starts, then the fixed-shape or general kernel) -> here:
-// 300,000 power-law rows, D = 128 bf16 196 -> 185 us, D = 64 fp32 170 -> 164; 100,000
+// 300,000 power-law rows, D = 128 bf16 196 -> 184 us, D = 64 fp32 170 -> 162; 100,000
 // lognormal rows, fp32, D = 16 / 32 17.9 -> 13.3, 24 -> 18; 85 204 -> 60; 40 84 -> 30;
 // 243,068 rows, D = 70 bf16 522 -> 79; 5000 rows, D = 64 19 -> 5.
 // U: 4, or 2 for 32-byte lanes on 8 lanes and more, which keeps 64 registers without
@@ -154,7 +154,10 @@ __global__ void __launch_bounds__(kCta, 4) sddmm_gather_kernel(
   const int g = lane / G, gl = lane & (G - 1);
   const unsigned w = blockIdx.x * (kCta / 32) + threadIdx.x / 32;
   if (w >= nblk) return;  // whole warp leaves together
-  const uint64_t pol = l2_policy_evict_normal();
+  // A row of X is read once, or for skewed rows by neighbouring warps: it leaves L2 to
+  // Y's rows, as the results do (300,000 power-law rows, D = 128 bf16 188 -> 184 us, D = 64
+  // fp32 167 -> 162; 400,000 rows of 16, D = 128 fp32 412 -> 404).
+  const uint64_t pol = l2_policy_evict_normal(), polx = l2_policy_evict_first();
   const unsigned pb = w * blk;
   const unsigned pe = nnz - pb < blk ? nnz : pb + blk;
   auto load_cols = [&](unsigned p) { return p + lane < pe ? ld_stream(col + (p + lane)) : 0; };
@@ -213,17 +216,18 @@ __global__ void __launch_bounds__(kCta, 4) sddmm_gather_kernel(
         const int left = FULL ? D : D - k0 - gl * E;
         const int chunks = left <= 0 ? 0 : imin(C, (left + G * E - 1) / (G * E));
         const size_t kb = FULL ? 0 : (size_t)(left > 0 ? k0 : 0) * sizeof(XT);
-        auto load = [&](const char *base, int r, unsigned ld, typename Dv::raw_t(&d)[C]) {
+        auto load = [&](const char *base, int r, unsigned ld, typename Dv::raw_t(&d)[C],
+                        uint64_t hint) {
           const XT *p_ = reinterpret_cast<const XT *>(base + (size_t)(unsigned)r * ld + kb);
 #pragma unroll
           for (int c = 0; c < C; ++c)
-            d[c] = FULL ? Dv::load(p_ + c * (G * E), pol)
-                        : Dv::load_if(p_ + c * (G * E), pol, c < chunks);
+            d[c] = FULL ? Dv::load(p_ + c * (G * E), hint)
+                        : Dv::load_if(p_ + c * (G * E), hint, c < chunks);
         };
         typename Dv::raw_t y[U][C];
 #pragma unroll
-        for (int u = 0; u < U; ++u) load(Yg, __shfl_sync(ALL, mc, t0 + u), ldy, y[u]);
-        if (r0 != xrow || (!FULL && D > G * E * C)) load(Xg, r0, ldx, xa);
+        for (int u = 0; u < U; ++u) load(Yg, __shfl_sync(ALL, mc, t0 + u), ldy, y[u], pol);
+        if (r0 != xrow || (!FULL && D > G * E * C)) load(Xg, r0, ldx, xa, polx);
         auto dot = [&](int u) {
 #pragma unroll
           for (int c = 0; c < C; ++c)
@@ -236,7 +240,7 @@ __global__ void __launch_bounds__(kCta, 4) sddmm_gather_kernel(
           for (int u = 0; u < U; ++u) dot(u);
         } else {
           typename Dv::raw_t xb[C];
-          load(Xg, r1, ldx, xb);
+          load(Xg, r1, ldx, xb, polx);
           int at = r0;
 #pragma unroll
           for (int u = 0; u < U; ++u) {
@@ -247,7 +251,7 @@ __global__ void __launch_bounds__(kCta, 4) sddmm_gather_kernel(
 #pragma unroll
                 for (int c = 0; c < C; ++c) xa[c] = xb[c];
               } else {
-                load(Xg, r, ldx, xa);
+                load(Xg, r, ldx, xa, polx);
               }
             }
             __syncwarp();
@@ -282,7 +286,7 @@ __global__ void __launch_bounds__(kCta, 4) sddmm_gather_kernel(
         }
       }
       const float v = __shfl_sync(ALL, mv, t0 + first);
-      if (owner && t0 + first < nb) out[p + (t0 + first)] = v * sum[0];
+      if (owner && t0 + first < nb) __stcs(out + (p + (t0 + first)), v * sum[0]);
     }
     mc = mcn;
     mv = mvn;
@@ -307,7 +311,8 @@ __device__ __forceinline__ void sddmm_fixed_block(
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int g = lane / G, gl = lane & (G - 1);
-  const uint64_t pol = l2_policy_evict_normal();
+  // (X as in sddmm_gather_kernel)
+  const uint64_t pol = l2_policy_evict_normal(), polx = l2_policy_evict_first();
   const long long pb = w * blk;
   const long long pe = pb + blk < nnz ? pb + blk : nnz;
   int mcn = pb + lane < pe ? ld_stream(col + pb + lane) : 0;
@@ -363,7 +368,7 @@ __device__ __forceinline__ void sddmm_fixed_block(
         if (row != xrow) {  // a new row for this group: its slice of X[i]
           const XT *xr = X + (long long)row * ldx + gl * V;
 #pragma unroll
-          for (int k = 0; k < KI; ++k) xa[k] = Dv::load(xr + k * G * V, pol);
+          for (int k = 0; k < KI; ++k) xa[k] = Dv::load(xr + k * G * V, polx);
           xrow = row;
         }
         const XT *yr = Y + (long long)j * ldy + gl * V;
@@ -381,7 +386,7 @@ __device__ __forceinline__ void sddmm_fixed_block(
       const float r = __shfl_sync(FULL, acc, ((lane - s * P) & (P - 1)) * G);
       if (lane / P == s) res = r;
     }
-    if (lane < nb) out[p + lane] = mv * res;
+    if (lane < nb) __stcs(out + (p + lane), mv * res);
   }
 }
 
