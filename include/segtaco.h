@@ -459,7 +459,9 @@ int segtaco_sddmm(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr, con
                                 4 elements (otherwise ignored) */
 typedef struct segtaco_sddmm_config {
   int32_t kernel;     /* SEGTACO_SDDMM_AUTO / _FIXED / _GENERAL / _BAND             */
-  int32_t block_nnz;  /* nonzeros per warp block, a power of two 32 .. 4096 (0: 256) */
+  int32_t block_nnz;  /* nonzeros per warp block, a power of two 32 .. 4096 (0: 256);
+                         with the automatic kernel and lanes the most that a warp
+                         takes: fewer where that fills the GPU's last wave     */
   int32_t lanes;      /* lanes per dot product (0: from D; power of two); a count
                          the fixed kernel has no shape for (one 32-byte load per
                          lane, two from 4 lanes, or four 16-byte loads) is

@@ -923,8 +923,7 @@ int segtaco_sddmm_ex(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr,
     if ((sh.family == 1 || sh.family == 2) && sh.KI == 2 && sh.G >= 8)
       return launch_sddmm(M, nnz, row_ptr, col, vals, X, Y, x_dtype, ldx, ldy, D, out, nullptr,
                           (int)P, nblk, s, false, 0, SEGTACO_SDDMM_FIXED);
-    return launch_sddmm_gather(M, nnz, row_ptr, col, vals, X, Y, x_dtype, ldx, ldy, D, out, (int)P,
-                               nblk, s);
+    return launch_sddmm_gather(M, nnz, row_ptr, col, vals, X, Y, x_dtype, ldx, ldy, D, out, (int)P, s);
   }
   Scratch scratch(nullptr, 0, s);
   SEGTACO_TRY(scratch.reserve(align256((size_t)(nblk + 1) * sizeof(int))));

@@ -216,8 +216,7 @@ int launch_sddmm_band(int M, int K, long long nnz, const int *row_ptr, const int
 bool sddmm_gather_applies(int x_dtype, long long ldx, long long ldy);
 int launch_sddmm_gather(int M, long long nnz, const int *row_ptr, const int *col,
                         const float *val, const void *X, const void *Y, int x_dtype,
-                        long long ldx, long long ldy, int D, float *out, int P, long long nblk,
-                        cudaStream_t s);
+                        long long ldx, long long ldy, int D, float *out, int P, cudaStream_t s);
 int launch_sddmm(int M, long long nnz, const int *row_ptr, const int *col, const float *val,
                  const void *X, const void *Y, int x_dtype, long long ldx, long long ldy, int D,
                  float *out, int *starts, int P, long long nblk, cudaStream_t s,

@@ -2,13 +2,14 @@
 //
 // segTACO's SDDMM (sddmm_csr_gpu_taco.h:5-150, CPU reference sddmm_csr_gpu.h:9-50)
 // is element-balanced: nonzero blocks with start rows from
-// taco_binarySearchBeforeBlock.  Here a warp takes a block of kSddmmBlock
-// nonzeros whose start row is the canonical block start; a group of G lanes
-// computes one dot product with V-wide loads of X[i] and Y[j] (one 16-byte load
-// per lane for D = 64 fp32 or D = 64 bf16), reduces it with xor shuffles, and
-// the 32 results of a batch leave in one coalesced store.  The loads of U = 4
-// steps (4P nonzeros) are issued before their multiply-adds.  X[i] is re-read
-// for every nonzero of row i but stays in L1.
+// taco_binarySearchBeforeBlock.  Here a warp takes a block of nonzeros (256 unless
+// the call says otherwise) and groups of G lanes one dot product each.  Three kernels:
+// the default (sddmm_gather_kernel, any D and alignment, its warps search their first
+// row), the fixed shapes (sddmm_fixed_kernel: D of 512 bytes and more in 32-byte
+// lanes, batches of problems, and explicit requests) and the general one
+// (sddmm_kernel: explicit requests and row pitches from 4 GB).
+#include <algorithm>
+#include <atomic>
 #include <climits>
 
 #include "common.cuh"
@@ -118,6 +119,13 @@ __global__ void __launch_bounds__(kCta, 3) sddmm_kernel(int M, long long nnz,
   }
 }
 
+// A row of X is read once, or for skewed rows by neighbouring warps: it leaves L2 to Y's
+// rows, as the results do.  Measured on GB300, X evict-normal / evict-first: 300,000
+// power-law rows, D = 128 bf16 187 / 184 us, D = 64 fp32 167 / 162; 200,000 rows of 16, D =
+// 128 fp32 155 / 150; where X and Y stay in L2 from call to call it costs up to 10 %
+// (90,862 rows of 16, D = 32 bf16 18.2 / 20.0), and a choice in the kernel costs the gain.
+__device__ __forceinline__ uint64_t sddmm_policy_x() { return l2_policy_evict_first(); }
+
 // The default kernel.  G lanes hold one dot product, each lane C chunks of E
 // elements (32 bytes where D, ldx, ldy and the pointers allow it, else 16, else one
 // or two elements), so the lanes of a group read whole lines of Y[j]; a group takes
@@ -154,10 +162,8 @@ __global__ void __launch_bounds__(kCta, 4) sddmm_gather_kernel(
   const int g = lane / G, gl = lane & (G - 1);
   const unsigned w = blockIdx.x * (kCta / 32) + threadIdx.x / 32;
   if (w >= nblk) return;  // whole warp leaves together
-  // A row of X is read once, or for skewed rows by neighbouring warps: it leaves L2 to
-  // Y's rows, as the results do (300,000 power-law rows, D = 128 bf16 188 -> 184 us, D = 64
-  // fp32 167 -> 162; 400,000 rows of 16, D = 128 fp32 412 -> 404).
-  const uint64_t pol = l2_policy_evict_normal(), polx = l2_policy_evict_first();
+  const uint64_t pol = l2_policy_evict_normal();
+  const uint64_t polx = sddmm_policy_x();
   const unsigned pb = w * blk;
   const unsigned pe = nnz - pb < blk ? nnz : pb + blk;
   auto load_cols = [&](unsigned p) { return p + lane < pe ? ld_stream(col + (p + lane)) : 0; };
@@ -311,8 +317,8 @@ __device__ __forceinline__ void sddmm_fixed_block(
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int g = lane / G, gl = lane & (G - 1);
-  // (X as in sddmm_gather_kernel)
-  const uint64_t pol = l2_policy_evict_normal(), polx = l2_policy_evict_first();
+  const uint64_t pol = l2_policy_evict_normal();
+  const uint64_t polx = sddmm_policy_x();
   const long long pb = w * blk;
   const long long pe = pb + blk < nnz ? pb + blk : nnz;
   int mcn = pb + lane < pe ? ld_stream(col + pb + lane) : 0;
@@ -423,6 +429,38 @@ __global__ void __launch_bounds__(kCta, 4) sddmm_fixed_multi_kernel(
                                   a.ldx, a.ldy, a.out, a.starts, w - a.blk_begin, kSddmmBlock);
 }
 
+// Blocks of at most P nonzeros per warp that fill whole waves of resident warps, so that
+// the last of a few waves is not nearly empty.  Measured on GB300, blocks of 256 /
+// here: rows of 16, 1.26M nonzeros (1.01 waves), D = 128 fp32 80 / 56 us, D = 64 51 / 35; 3.2M
+// (2.6 waves), D = 128 163 / 150; 1.8M lognormal (1.5 waves), D = 100 113 / 97; 60,000
+// power-law rows (1.1 waves), D = 64 47 / 39; from four waves on it makes no difference.
+struct SddmmGrid {
+  long long blk, nblk;
+  unsigned ctas;
+};
+template <auto Kernel> SddmmGrid sddmm_grid(long long nnz, int P) {
+  static std::atomic<int> per_sm{0};
+  int n = per_sm.load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, Kernel, kCta, 0) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = 4;
+    }
+    per_sm.store(n, std::memory_order_relaxed);
+  }
+  const long long slots = (long long)device_sms() * n * (kCta / 32);
+  const long long waves = (nnz + P * slots - 1) / (P * slots);
+  SddmmGrid g;
+  g.blk = P;
+  if (waves > 1 && waves <= 4) {
+    const long long each = (nnz + waves * slots - 1) / (waves * slots);
+    g.blk = std::min<long long>(P, (each + 15) / 16 * 16);
+  }
+  g.nblk = (nnz + g.blk - 1) / g.blk;
+  g.ctas = (unsigned)((g.nblk + kCta / 32 - 1) / (kCta / 32));
+  return g;
+}
+
 // Fixed shapes (KI, G) of each family, for both launches.
 #define SEGTACO_SDDMM_SHAPES32(X_) \
   X_(1, 1) X_(1, 2) X_(1, 4) X_(2, 4) X_(2, 8) X_(2, 16) X_(1, 8) X_(1, 16) X_(1, 32)
@@ -509,10 +547,13 @@ int launch_fixed_single(const SddmmShape &sh, int x_dtype, dim3 grid, int M, lon
                         const void *Y, long long ldx, long long ldy, float *out, const int *starts,
                         long long nblk, int blk, cudaStream_t s) {
 #define CASE_(XT, V, KI, G)                                                                \
-  sddmm_fixed_kernel<XT, V, G, KI><<<grid, kCta, 0, s>>>(M, nnz, row_ptr, col, val,       \
-                                                         static_cast<const XT *>(X),      \
-                                                         static_cast<const XT *>(Y), ldx, \
-                                                         ldy, out, starts, nblk, blk);
+  {                                                                                        \
+    SddmmGrid b{blk, nblk, grid.x};                                                        \
+    if (!starts) b = sddmm_grid<&sddmm_fixed_kernel<XT, V, G, KI>>(nnz, blk);              \
+    sddmm_fixed_kernel<XT, V, G, KI><<<b.ctas, kCta, 0, s>>>(                              \
+        M, nnz, row_ptr, col, val, static_cast<const XT *>(X), static_cast<const XT *>(Y), ldx, \
+        ldy, out, starts, b.nblk, (int)b.blk);                                             \
+  }
   SEGTACO_SDDMM_SWITCH(sh, x_dtype)
 #undef CASE_
   return check_launch("sddmm_fixed_kernel");
@@ -547,20 +588,23 @@ int launch_fixed_multi(const SddmmShape &sh, int x_dtype, dim3 grid, const Sddmm
   X_(XT, E, 1, 1) X_(XT, E, 1, 2) X_(XT, E, 1, 4) X_(XT, E, 1, 8) X_(XT, E, 1, 16) X_(XT, E, 1, 32)
 #define SEGTACO_SDDMM_KEY(E, C, G) ((E)*10000 + (C)*100 + (G))
 #define SEGTACO_SDDMM_RUN(XT, E, C, G, F)                                                  \
-  sddmm_gather_kernel<XT, E, C, G, F><<<grid, kCta, 0, s>>>(                               \
-      M, (unsigned)nnz, row_ptr, col, val, static_cast<const XT *>(X),                     \
-      static_cast<const XT *>(Y), (unsigned)(ldx * sizeof(XT)), (unsigned)(ldy * sizeof(XT)), D, \
-      out, (unsigned)nblk, (unsigned)P)
+  {                                                                                        \
+    const SddmmGrid b = sddmm_grid<&sddmm_gather_kernel<XT, E, C, G, F>>(nnz, P);          \
+    sddmm_gather_kernel<XT, E, C, G, F><<<b.ctas, kCta, 0, s>>>(                           \
+        M, (unsigned)nnz, row_ptr, col, val, static_cast<const XT *>(X),                   \
+        static_cast<const XT *>(Y), (unsigned)(ldx * sizeof(XT)), (unsigned)(ldy * sizeof(XT)), \
+        D, out, (unsigned)b.nblk, (unsigned)b.blk);                                        \
+  }
 #define SEGTACO_SDDMM_NARROW_CASE(XT, E, C, G)  \
   case SEGTACO_SDDMM_KEY(E, C, G):              \
-    SEGTACO_SDDMM_RUN(XT, E, C, G, false);      \
+    SEGTACO_SDDMM_RUN(XT, E, C, G, false)       \
     break;
 #define SEGTACO_SDDMM_WIDE_CASE(XT, E, C, G)    \
   case SEGTACO_SDDMM_KEY(E, C, G):              \
     if (D == (E) * (C) * (G))                   \
-      SEGTACO_SDDMM_RUN(XT, E, C, G, true);     \
+      SEGTACO_SDDMM_RUN(XT, E, C, G, true)      \
     else                                        \
-      SEGTACO_SDDMM_RUN(XT, E, C, G, false);    \
+      SEGTACO_SDDMM_RUN(XT, E, C, G, false)     \
     break;
 
 bool sddmm_gather_applies(int x_dtype, long long ldx, long long ldy) {
@@ -570,9 +614,8 @@ bool sddmm_gather_applies(int x_dtype, long long ldx, long long ldy) {
 
 int launch_sddmm_gather(int M, long long nnz, const int *row_ptr, const int *col,
                         const float *val, const void *X, const void *Y, int x_dtype,
-                        long long ldx, long long ldy, int D, float *out, int P, long long nblk,
+                        long long ldx, long long ldy, int D, float *out, int P,
                         cudaStream_t s) {
-  const dim3 grid((unsigned)((nblk + (kCta / 32) - 1) / (kCta / 32)));
   const int esz = x_dtype == SEGTACO_BF16 ? 2 : 4;
   const uintptr_t al = (uintptr_t)X | (uintptr_t)Y;
   int E = 32 / esz;

@@ -64,3 +64,26 @@ def test_rows_outside_the_pattern_stay_out(cuda, D):
     want = ops.sddmm(dev(A), Xd, Yd)
     Yd[0, ::2], Yd[0, 1::2] = float("inf"), float("nan")
     assert torch.equal(ops.sddmm(dev(A), Xd, Yd), want)
+
+
+@pytest.mark.parametrize("nnz", [1_250_003, 2_600_017])
+@pytest.mark.parametrize("per_row", [1, 16, 33])
+@pytest.mark.parametrize("D,bf16", [(5, False), (64, False), (64, True), (128, False)])
+def test_blocks_fitted_to_the_waves(cuda, D, bf16, per_row, nnz):
+    """From one to four waves of warps a block is not a power of two, and the last one is short."""
+    M, K = (nnz + per_row - 1) // per_row, 500
+    rng = np.random.default_rng(3)
+    A = synth.CSR(np.minimum(np.arange(M + 1) * per_row, nnz).astype(np.int32),
+                  rng.integers(0, K, nnz).astype(np.int32),
+                  rng.standard_normal(nnz).astype(np.float32), M, K)
+    X, Y = (torch.randn(n, D, device="cuda", dtype=torch.bfloat16 if bf16 else torch.float32)
+            for n in (M, K))
+    Ad = dev(A)
+    out = ops.sddmm(Ad, X, Y, out=torch.full((nnz,), float("nan"), device="cuda"))
+    rows, cols = torch.arange(nnz, device="cuda") // per_row, Ad.col.long()
+    for p in range(0, nnz, 1 << 18):
+        q = slice(p, min(p + (1 << 18), nnz))
+        xy = X[rows[q]].double() * Y[cols[q]].double()
+        v = Ad.val[q].double()
+        err = (out[q].double() - v * xy.sum(1)).abs()
+        assert (err <= TOL * v.abs() * xy.abs().sum(1) + 1e-30).all(), err.max()
