@@ -244,7 +244,8 @@ int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, lo
   if (c.depth != 0 && c.depth != 4 && c.depth != 8)
     return set_error(SEGTACO_EINVAL, "depth=%d not in {0, 4, 8}", c.depth);
   plan->deep = c.depth == 8;
-  // Walk: the flat walk by default for eb_sr (one slot over merge-path chunks:
+  // Walk, where neither the split walk nor row slots nor joined chunks apply (below):
+  // the flat walk by default for eb_sr (one slot over merge-path chunks:
   // short rows share a batch of 32 nonzeros instead of a round trip each;
   // measured on GB300 1.44 vs 1.53 ms on the 1M x 1M power-law SpMM), the row
   // walk everywhere else (rb units are too small to amortise the flat walk's
@@ -612,7 +613,7 @@ int segtaco_autotune_heuristic(int32_t M, int32_t K, int64_t nnz, int32_t N, int
   // Pieces / joined chunks, power-law rows: 60,000, N = 64 108 / 45, 400,000, N = 37 432 /
   // 183, N = 128 372 / 420 fp32 and 301 / 274 bf16; 400,000 lognormal rows, N = 128 395 / 278.
   const bool join = schedule == SEGTACO_RB_PR && !even && !(heavy && esz == 4 && N % 8 == 0) &&
-                    (long_rows || (nnz < kLongRowsMinNnz && max_row_len >= 640 &&
+                    (long_rows || (nnz < kLongRowsMinNnz && max_row_len >= kJoinRow &&
                                    !(banded && N >= 64 && N % 16 == 0)));
   // A B that fits L2 whole (up to ~96 MB) under a large product: one slab of
   // up to 64 columns (8 per lane, G = 8), so A is read once.  Measured on
@@ -710,6 +711,11 @@ int segtaco_spmm_workspace_size(int32_t M, int32_t K, int64_t nnz, int32_t N, in
   return SEGTACO_OK;
 }
 
+// Whether a caller's workspace holds the sums of joined chunks.
+static bool holds_sums(const SpmmPlan &plan, const void *workspace, size_t bytes) {
+  return bytes >= plan.workspace && ((uintptr_t)workspace & 255) == 0;
+}
+
 int segtaco_spmm(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr, const int32_t *col,
                  const float *vals, const void *B, int32_t b_dtype, int64_t ldb, float *C,
                  int64_t ldc, int32_t N, const segtaco_config *cfg, void *workspace,
@@ -724,8 +730,8 @@ int segtaco_spmm(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr, cons
   if (ldb < N || ldc < N) return set_error(SEGTACO_EINVAL, "ldb/ldc smaller than N");
   SpmmPlan plan;
   SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, ldb, ldc, B, C, cfg, &plan));
-  // A caller's workspace without room for the sums of cut rows: the pieces or row blocks
-  if (plan.walk == kWalkSplitJoin && workspace && workspace_bytes < plan.workspace)
+  // A caller's workspace that cannot hold the sums of cut rows: the pieces or row blocks
+  if (plan.walk == kWalkSplitJoin && workspace && !holds_sums(plan, workspace, workspace_bytes))
     SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, ldb, ldc, B, C, cfg, &plan,
                           LongRowScratch::kPieces));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -739,7 +745,9 @@ int segtaco_spmm(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr, cons
     px = static_cast<int *>(scratch.take(plan.px_entries * sizeof(int)));
     py = static_cast<int *>(scratch.take(plan.py_entries * sizeof(int)));
   }
-  if (ready && plan.workspace && !workspace && plan.walk != kWalkSplitJoin)
+  // (below the pieces' size rb_pr has nothing prepared and needs no caller's workspace)
+  if (ready && plan.workspace && !workspace &&
+      (plan.walk != kWalkSplitJoin || nnz >= kLongRowsMinNnz))
     return set_error(SEGTACO_EINVAL, "PARTITION_READY needs the caller's workspace");
   return run_spmm_planned(plan, M, K, nnz, row_ptr, col, vals, B, b_dtype, ldb, C, ldc, N, px, py,
                           s, ready);
@@ -753,7 +761,7 @@ int segtaco_spmm_partition(int32_t M, int32_t K, int64_t nnz, const int32_t *row
   if (C == nullptr || ldc < N) return set_error(SEGTACO_EINVAL, "C is NULL or ldc < N");
   SpmmPlan plan;
   SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, N, ldc, nullptr, C, cfg, &plan));
-  if (plan.walk == kWalkSplitJoin && workspace_bytes >= plan.workspace)
+  if (plan.walk == kWalkSplitJoin && workspace && holds_sums(plan, workspace, workspace_bytes))
     return SEGTACO_OK;  // nothing to prepare
   if (plan.walk == kWalkSplitJoin)
     SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, N, ldc, nullptr, C, cfg, &plan,

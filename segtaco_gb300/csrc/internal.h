@@ -164,6 +164,9 @@ struct SpmmPlan {
   long long py_entries;      // ... of the second (eb: chunk-edge nonzeros; long rows: counters)
   size_t workspace;          // bytes
 };
+// rb_pr below 1M nonzeros: a longest row of this many calls for joined chunks (measured
+// in segtaco_autotune_heuristic).
+constexpr int kJoinRow = 640;
 // What the workspace has room for under rb_pr's long rows: the sums of joined chunks
 // (spmm_join.cu), else pieces, else the list of the long-row CTAs, as for rb_sr.
 enum class LongRowScratch { kList, kPieces, kJoin };

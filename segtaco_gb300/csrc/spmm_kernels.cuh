@@ -36,6 +36,11 @@
 // row is written once with a plain store, so C needs no memset and atomics
 // happen only at partition edges.
 //
+// By default chunks of up to 512 items take the split walk instead (spmm_split.cuh),
+// row blocks of even rows the row slots (spmm_rows.cuh) and rb_pr's uneven rows joined
+// chunks (spmm_join.cu).  The walks here serve rb_sr's uneven rows, rb_pr's short
+// uneven ones and its pieces, fp32's 32-byte lanes, and explicit requests.
+//
 // Blocks of the grid are dispatched x-fastest, so the GPU finishes (roughly)
 // slab 0 of all units before slab 1: only a K x W slab of B has to stay in L2.
 #pragma once

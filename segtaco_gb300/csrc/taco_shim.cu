@@ -445,8 +445,20 @@ int run_spmm(const Entry &e, taco_tensor_t *C, taco_tensor_t *A, taco_tensor_t *
     cfg.items_per_unit = e.items;
     cfg.col_tile = e.col_tile;
     // Row-block names: long rows out of the row blocks (rb_sr: CTAs of their
-    // own; rb_pr: pieces) when the host CSR has any.
-    if ((e.schedule == SEGTACO_RB_SR || e.schedule == SEGTACO_RB_PR) && nnz >= segtaco::kLongRowsMinNnz) {
+    // own; rb_pr: joined chunks, or with explicit lanes or a threshold pieces) when
+    // the host CSR has any.  Measured on GB300, spmm_rb_pr calls on pageable operands,
+    // power-law rows: 20,000, N = 37 1025 -> 130 us, 40,000, N = 64 1587 -> 246.
+    if (e.schedule == SEGTACO_RB_PR && cfg.items_per_unit <= 0 && cfg.vec == 0 &&
+        cfg.rows_per_unit <= 1) {
+      const int T = nnz >= segtaco::kLongRowsMinNnz ? (int)segtaco::kPieceThreshold : segtaco::kJoinRow;
+      int longest = 0;
+      for (int r0 = 0; r0 < M && longest < T; r0 += 4096)
+        for (int r = r0; r < std::min(M, r0 + 4096); ++r) longest = std::max(longest, rp[r + 1] - rp[r]);
+      if (longest >= T) {
+        cfg.flags |= SEGTACO_FLAG_LONG_ROWS;
+        cfg.depth = 8;
+      }
+    } else if ((e.schedule == SEGTACO_RB_SR || e.schedule == SEGTACO_RB_PR) && nnz >= segtaco::kLongRowsMinNnz) {
       const long long T = e.schedule == SEGTACO_RB_PR && cfg.items_per_unit <= 0
                               ? segtaco::kPieceThreshold
                               : segtaco::long_row_threshold(cfg);

@@ -66,6 +66,8 @@ def test_workspaces_and_capture(cuda):
         ops.spmm_partition(Ad, C2, _cfg(), ws)
         ops.spmm(Ad, Bd, C2, ready, ws)
         assert torch.equal(C, C2)
+    with pytest.raises(Exception, match="needs the caller's workspace"):
+        ops.spmm(Ad, Bd, _nan(A, n), ready)
     with pytest.raises(Exception, match="workspace too small"):
         ops.spmm(Ad, Bd, _nan(A, n), _cfg(), torch.empty(256, dtype=torch.uint8, device="cuda"))
     C = _nan(A, n)
@@ -88,8 +90,9 @@ def test_small_products_need_no_workspace(cuda):
     B = synth.dense(A.K, 24, seed=5)
     Ad, Bd = dev(A), torch.from_numpy(B).cuda()
     ws = torch.empty(256, dtype=torch.uint8, device="cuda")
+    odd = torch.empty(1 << 20, dtype=torch.uint8, device="cuda")[4:]  # not 256-byte aligned
     ops.spmm_partition(Ad, _nan(A, 24), _cfg(), ws)
-    for C in (ops.spmm(Ad, Bd, _nan(A, 24), _cfg(), ws),
+    for C in (ops.spmm(Ad, Bd, _nan(A, 24), _cfg(), ws), ops.spmm(Ad, Bd, _nan(A, 24), _cfg(), odd),
               ops.spmm(Ad, Bd, _nan(A, 24), _cfg(N.FLAG_PARTITION_READY))):
         assert_spmm_close(C.cpu().numpy(), A, B)
 
