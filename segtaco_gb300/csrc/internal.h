@@ -229,16 +229,17 @@ int launch_sddmm(int M, long long nnz, const int *row_ptr, const int *col, const
 // Row-block products below this many nonzeros walk every row in the row-block
 // kernel: the list pass and the fork would cost more than a long row there.
 constexpr long long kLongRowsMinNnz = 1000000;
-// Merge-path items per chunk of a product launched alone: 512 (a warp's
-// chunk), halved down to 32 while the grid would hold fewer than 3,072
-// chunks, so that small products still fill the 152 SMs.  Measured on GB300
-// (partition + product, split walk): 77,777 lognormal rows (1.02M items), N = 32,
-// 128 / 256 / 512 items 21.5 / 19.6 / 23.7 us; 20,000 rows (263K), N = 16, 64 /
-// 128 / 256 items 10.0 / 11.2 / 12.6 us.
+// Merge-path items per chunk of a product launched alone: one wave of 152 x 32 warps
+// (the split walk holds 32 to 36 per SM), in steps of 16, at least 32 and at most 512.
+// Measured on GB300, split walk, a power of two with 3,072 chunks and more / one wave:
+// 90,000 rows of 16 (1.5M items), N = 64 38.2 / 30.1 us (256, 320); 60,000 power-law rows,
+// N = 64 39.4 / 33.5; 130,000 lognormal rows, N = 64 40.4 / 35.2 (512, 352), 60,000, N = 32
+// 19.4 / 16.3, 30,000, N = 128 24.3 / 20.2 (64, 96).  Beyond 512 items the chunk stays:
+// 250,000 power-law rows (5.2M items), N = 64 108 us with 512, 113 with three full waves of
+// 368.
 inline long long default_chunk_items(long long M, long long nnz) {
-  long long D = 512;
-  while (D > 32 && (M + nnz) / D < 3072) D >>= 1;
-  return D;
+  const long long D = (M + nnz + 152 * 32 - 1) / (152 * 32);
+  return D < 32 ? 32 : D > 512 ? 512 : (D + 15) / 16 * 16;
 }
 // Default long-row threshold (items_per_unit = 0).  Measured on GB300 (1M x 1M
 // power law, N = 128, Zipf 1.8 / 1.922, rb_sr): 1024: 2.33 / 1.45 ms, 2048:
