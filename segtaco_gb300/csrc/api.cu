@@ -639,7 +639,12 @@ int segtaco_autotune_heuristic(int32_t M, int32_t K, int64_t nnz, int32_t N, int
   if (schedule == SEGTACO_RB_SR)
     while (cfg->rows_per_unit > 1 && M / cfg->rows_per_unit < 8192) cfg->rows_per_unit >>= 1;
   // rb: 8 loads in flight in the row walk, or (4) even rows side by side.
-  cfg->depth = (schedule == SEGTACO_RB_SR || schedule == SEGTACO_RB_PR) && !even ? 8 : 4;
+  // (rb_pr's rows of more than 32 nonzeros in 16-byte lanes stay with the row walk;
+  // 8 with long rows would ask for joined chunks, even rows keep the pieces.)
+  const bool side_by_side =
+      even &&
+      (schedule == SEGTACO_RB_SR || nnz <= 32LL * M || N % (16 / esz) != 0 || long_rows);
+  cfg->depth = (schedule == SEGTACO_RB_SR || schedule == SEGTACO_RB_PR) && !side_by_side ? 8 : 4;
   cfg->flags = long_rows || join ? SEGTACO_FLAG_LONG_ROWS : 0;
   // rb_pr's long rows as pieces of the row-block launch (rows of >= 512
   // nonzeros, pieces of 4096); the rows left are short, so a warp takes 64 of
