@@ -6,17 +6,25 @@
 
 namespace segtaco {
 
-// x = hi + mid + lo for two values, each part a bf16 pair (truncation: exact).
+// x = hi + mid + lo for two values, each part a bf16 pair, rounded to nearest, so that
+// |mid| <= 2^-8 and |lo| <= 2^-17 of x's leading bit and neither has x's sign for good: the
+// products of mid and lo that a caller leaves out are below 2^-24 of the whole and
+// cancel (cut off instead, mid and lo reach 2^-7 and 2^-15, all one way: up to 4.7e-7
+// of a product).  Values from the middle between bf16's largest and 2^128 on give
+// infinite and NaN parts, as infinities and NaN do.
+__device__ __forceinline__ uint32_t round_bf16x2(float x, float y) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+  return r;
+}
 __device__ __forceinline__ void split3(float x, float y, uint32_t &hi, uint32_t &mid,
                                        uint32_t &lo) {
-  const uint32_t xb = __float_as_uint(x), yb = __float_as_uint(y);
-  hi = __byte_perm(xb, yb, 0x7632);
-  const float xr = x - __uint_as_float(xb & 0xffff0000u);
-  const float yr = y - __uint_as_float(yb & 0xffff0000u);
-  const uint32_t xm = __float_as_uint(xr), ym = __float_as_uint(yr);
-  mid = __byte_perm(xm, ym, 0x7632);
-  lo = __byte_perm(__float_as_uint(xr - __uint_as_float(xm & 0xffff0000u)),
-                   __float_as_uint(yr - __uint_as_float(ym & 0xffff0000u)), 0x7632);
+  hi = round_bf16x2(x, y);
+  const float xr = x - __uint_as_float(hi << 16);
+  const float yr = y - __uint_as_float(hi & 0xffff0000u);
+  mid = round_bf16x2(xr, yr);
+  lo = __byte_perm(__float_as_uint(xr - __uint_as_float(mid << 16)),
+                   __float_as_uint(yr - __uint_as_float(mid & 0xffff0000u)), 0x7632);
 }
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
                                          uint32_t b1) {

@@ -9,10 +9,10 @@
 // tile <X[i0 + r], Y[jw0 + j]> of its 32 rows and the 32 + 2 kSbHalo window rows
 // around the diagonal (column i0 * K / M of its first row), a 32 x 96 x 64
 // contraction that runs as mma.m16n8k16 with fp32 accumulation.  bf16 factors take one
-// product per step.  fp32 factors are cut exactly into three bf16 parts (hi + mid +
-// lo, 8 bits each) and the six products down to 2^-16 of the largest are summed per
-// step of 16 elements, the smallest first, then added to the running sum in fp32; what
-// is left out is below 2^-24 of a product.  Warp w takes window rows 24 w .. +23 and
+// product per step.  fp32 factors are split into three bf16 parts (hi + mid + lo, rounded
+// to nearest: mma.cuh) and six of the nine products summed per step of 16 elements,
+// hi x hi by itself and the others the smallest first, both then added to the running
+// sum in fp32; what is left out is below 2^-24 of a product, either way.  Warp w takes window rows 24 w .. +23 and
 // all 32 rows; a lane's four elements of a row are one load of 16 (8) bytes, in the
 // same order for X and Y, so neither needs transposing or, for Y, shared memory.  The
 // tile then goes to shared memory and every nonzero of the block reads its dot product
@@ -20,8 +20,9 @@
 // computed by 16 lanes each, 4 elements per lane from the X block and Y[j] in global
 // memory, summed by shuffles; beyond the list a thread computes the dot product alone.
 // The tile holds dot products for window positions without a nonzero too (96 per row
-// instead of ~2 kSbHalo + 1).  Splitting an infinity or NaN would make NaN of both: a
-// CTA that meets one in fp32 factors computes its dot products one by one instead.
+// instead of ~2 kSbHalo + 1).  Splitting an infinity or NaN makes NaN of both, and a
+// value next to the largest splits into infinite parts: a CTA with fp32 factors whose
+// tile holds any such sum computes its dot products one by one instead.
 //
 // What bounds it: the sampling of the tile and the off-band gathers, each about half
 // of what the product leaves (without the off-band list 136 us, without the product
@@ -30,6 +31,8 @@
 // bf16 222 -> 150; error against FP64 1.4e-7 -> 9.7e-8 and 5.0e-8 -> 4.6e-8.  Eight
 // off-band steps in flight instead of four 206 -> 195 us; 20 sampled nonzeros in flight
 // instead of 10 spill (258); a warp per row in the sampling 252.
+#include <cfloat>
+
 #include "common.cuh"
 #include "internal.h"
 #include "mma.cuh"
@@ -111,7 +114,6 @@ __global__ void __launch_bounds__(kSbCta, sizeof(XT) == 4 ? 5 : 6)  // 96 / 80 r
   for (int m = 0; m < 2; ++m)
 #pragma unroll
     for (int n = 0; n < 3; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.0f;
-  float amax = 0.0f;  // the factors' largest magnitude, or NaN
 #pragma unroll 1
   for (int s = 0; s < kSbD / 16; ++s) {
     float4 ynext[3];
@@ -124,7 +126,6 @@ __global__ void __launch_bounds__(kSbCta, sizeof(XT) == 4 ? 5 : 6)  // 96 / 80 r
       uint32_t(&p)[kParts][4] = xa[h >> 1];
       const int q = h & 1;  // registers q (elements 0, 1) and q + 2 (elements 2, 3)
       if constexpr (kSplit) {
-        amax = max_nan(max_nan(max_nan(max_nan(amax, x.x), x.y), x.z), x.w);
         split3(x.x, x.y, p[0][q], p[1][q], p[2][q]);
         split3(x.z, x.w, p[0][q + 2], p[1][q + 2], p[2][q + 2]);
       } else {
@@ -137,7 +138,6 @@ __global__ void __launch_bounds__(kSbCta, sizeof(XT) == 4 ? 5 : 6)  // 96 / 80 r
       uint32_t yb[kParts][2];
       const float4 y = ycur[n];
       if constexpr (kSplit) {
-        amax = max_nan(max_nan(max_nan(max_nan(amax, y.x), y.y), y.z), y.w);
         split3(y.x, y.y, yb[0][0], yb[1][0], yb[2][0]);
         split3(y.z, y.w, yb[0][1], yb[1][1], yb[2][1]);
       } else {
@@ -147,15 +147,16 @@ __global__ void __launch_bounds__(kSbCta, sizeof(XT) == 4 ? 5 : 6)  // 96 / 80 r
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
         float d[4];
+        mma_bf16_zero(d, xa[m][0], yb[0][0], yb[0][1]);  // hi hi
         if constexpr (kSplit) {
-          mma_bf16_zero(d, xa[m][0], yb[2][0], yb[2][1]);  // hi lo
-          mma_bf16(d, xa[m][2], yb[0][0], yb[0][1]);       // lo hi
-          mma_bf16(d, xa[m][1], yb[1][0], yb[1][1]);       // mid mid
-          mma_bf16(d, xa[m][0], yb[1][0], yb[1][1]);       // hi mid
-          mma_bf16(d, xa[m][1], yb[0][0], yb[0][1]);       // mid hi
-          mma_bf16(d, xa[m][0], yb[0][0], yb[0][1]);       // hi hi
-        } else {
-          mma_bf16_zero(d, xa[m][0], yb[0][0], yb[0][1]);
+          float e[4];
+          mma_bf16_zero(e, xa[m][0], yb[2][0], yb[2][1]);  // hi lo
+          mma_bf16(e, xa[m][2], yb[0][0], yb[0][1]);       // lo hi
+          mma_bf16(e, xa[m][1], yb[1][0], yb[1][1]);       // mid mid
+          mma_bf16(e, xa[m][0], yb[1][0], yb[1][1]);       // hi mid
+          mma_bf16(e, xa[m][1], yb[0][0], yb[0][1]);       // mid hi
+#pragma unroll
+          for (int q = 0; q < 4; ++q) d[q] += e[q];
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[m][n][q] += d[q];
@@ -185,8 +186,13 @@ __global__ void __launch_bounds__(kSbCta, sizeof(XT) == 4 ? 5 : 6)  // 96 / 80 r
       *reinterpret_cast<float2 *>(dst) = make_float2(acc[m][n][0], acc[m][n][1]);
       *reinterpret_cast<float2 *>(dst + 8 * kSbTP) = make_float2(acc[m][n][2], acc[m][n][3]);
     }
-  // An infinity or NaN among fp32 factors: every dot product by itself.
-  const bool direct = __syncthreads_or(kSplit && !(fabsf(amax) <= 3.402823466e38f)) != 0;
+  // An infinity or NaN among the tile's sums: every dot product by itself.
+  float amax = 0.0f;
+  if constexpr (kSplit) {
+#pragma unroll
+    for (int q = 0; q < 24; ++q) amax = max_nan(amax, acc[q / 12][q / 4 % 3][q % 4]);
+  }
+  const bool direct = __syncthreads_or(kSplit && !(fabsf(amax) <= FLT_MAX)) != 0;
   // The block's nonzeros, coalesced, kSq per thread per pass.
   for (int n0 = t; n0 < len; n0 += SQ * kSbCta) {
     if (n0 != t) load_nz(n0);
