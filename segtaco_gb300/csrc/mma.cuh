@@ -43,6 +43,16 @@ __device__ __forceinline__ void mma_bf16_zero(float (&d)[4], const uint32_t (&a)
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
 }
+// Smallest nonzero magnitude: the smaller of `least` (start: 0xffffffff) and twice x's
+// bits less one (zeros wrap to the top).  Below kSplitMin the parts of a value can fall
+// under bf16's smallest normal number, 2^-126, where the last bits of `lo` are lost or left
+// to the tensor cores' treatment of subnormals; a kernel that splits sends such values
+// another way.
+constexpr uint32_t kSplitMin = 2u * ((127u - 103u) << 23) - 1u;  // |x| = 2^-103
+__device__ __forceinline__ uint32_t min_nonzero(uint32_t least, float x) {
+  const uint32_t b = __float_as_uint(x);
+  return min(least, b + b - 1u);
+}
 // The larger magnitude (its sign is no use), NaN if either is NaN.
 __device__ __forceinline__ float max_nan(float a, float b) {
   float r;

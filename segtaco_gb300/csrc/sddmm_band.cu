@@ -21,8 +21,9 @@
 // memory, summed by shuffles; beyond the list a thread computes the dot product alone.
 // The tile holds dot products for window positions without a nonzero too (96 per row
 // instead of ~2 kSbHalo + 1).  Splitting an infinity or NaN makes NaN of both, and a
-// value next to the largest splits into infinite parts: a CTA with fp32 factors whose
-// tile holds any such sum computes its dot products one by one instead.
+// value next to the largest splits into infinite parts; one below 2^-103 has no three
+// parts.  A CTA with fp32 factors that meets such a sum or value computes its dot
+// products one by one instead.
 //
 // What bounds it: the sampling of the tile and the off-band gathers, each about half
 // of what the product leaves (without the off-band list 136 us, without the product
@@ -91,6 +92,11 @@ __global__ void __launch_bounds__(kSbCta, sizeof(XT) == 4 ? 5 : 6)  // 96 / 80 r
     yok[n] = j >= 0 && j < K;
     yrow[n] = Y + (size_t)(yok[n] ? j : 0) * ldy + e4;
   }
+  uint32_t least = 0xffffffffu;  // the fp32 factors' smallest nonzero magnitude
+  auto note = [&](const float4 &v) {
+    if constexpr (kSplit)
+      least = min_nonzero(min_nonzero(min_nonzero(min_nonzero(least, v.x), v.y), v.z), v.w);
+  };
   auto load_y = [&](int s, float4(&y)[3]) {
 #pragma unroll
     for (int n = 0; n < 3; ++n)
@@ -102,8 +108,10 @@ __global__ void __launch_bounds__(kSbCta, sizeof(XT) == 4 ? 5 : 6)  // 96 / 80 r
   for (int u = 0; u < 4; ++u) {
     const int e = t + u * kSbCta;  // 0 .. 511: row e / 16, elements 4 (e % 16) ..
     const int i = i0 + e / (kSbD / 4);
-    *reinterpret_cast<float4 *>(xr + (e / (kSbD / 4)) * kSbXP + 4 * (e % (kSbD / 4))) =
+    const float4 x =
         i < M ? sb_ld4<XT>(X + (size_t)i * ldx + 4 * (e % (kSbD / 4))) : make_float4(0, 0, 0, 0);
+    *reinterpret_cast<float4 *>(xr + (e / (kSbD / 4)) * kSbXP + 4 * (e % (kSbD / 4))) = x;
+    note(x);
   }
   if (t <= kSbRows) rp[t] = __ldg(row_ptr + min(i0 + t, M));
   if (t == 0) lcount = 0;
@@ -137,6 +145,7 @@ __global__ void __launch_bounds__(kSbCta, sizeof(XT) == 4 ? 5 : 6)  // 96 / 80 r
     for (int n = 0; n < 3; ++n) {
       uint32_t yb[kParts][2];
       const float4 y = ycur[n];
+      note(y);
       if constexpr (kSplit) {
         split3(y.x, y.y, yb[0][0], yb[1][0], yb[2][0]);
         split3(y.z, y.w, yb[0][1], yb[1][1], yb[2][1]);
@@ -186,13 +195,13 @@ __global__ void __launch_bounds__(kSbCta, sizeof(XT) == 4 ? 5 : 6)  // 96 / 80 r
       *reinterpret_cast<float2 *>(dst) = make_float2(acc[m][n][0], acc[m][n][1]);
       *reinterpret_cast<float2 *>(dst + 8 * kSbTP) = make_float2(acc[m][n][2], acc[m][n][3]);
     }
-  // An infinity or NaN among the tile's sums: every dot product by itself.
+  // An infinity or NaN among the tile's sums, or a tiny factor: every dot product by itself.
   float amax = 0.0f;
   if constexpr (kSplit) {
 #pragma unroll
     for (int q = 0; q < 24; ++q) amax = max_nan(amax, acc[q / 12][q / 4 % 3][q % 4]);
   }
-  const bool direct = __syncthreads_or(kSplit && !(fabsf(amax) <= FLT_MAX)) != 0;
+  const bool direct = __syncthreads_or(kSplit && (!(fabsf(amax) <= FLT_MAX) || least < kSplitMin)) != 0;
   // The block's nonzeros, coalesced, kSq per thread per pass.
   for (int n0 = t; n0 < len; n0 += SQ * kSbCta) {
     if (n0 != t) load_nz(n0);

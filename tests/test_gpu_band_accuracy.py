@@ -50,3 +50,27 @@ def test_sddmm_equal_factors(cuda):
     X = np.full((A.M, D), 1 + 2.0 ** -7 - 2.0 ** -23, np.float32)
     out, want, bound = _sddmm(A, X, X)
     assert (np.abs(out - want) <= 1.02 * 3.25 * 2.0 ** -24 * bound).all()
+
+
+@pytest.mark.parametrize("sx,sy", [(1e-36, 1e30), (1e-30, 1e-3), (1e30, 1e-37), (1e-20, 1e-18), (1e-39, 1e38),
+                                   (3e-19, 3e-19), (1e-44, 1e38)])
+def test_sddmm_small_magnitudes(cuda, sx, sy):
+    """Dot products as near as 68 fp32 operations bring them (2^-24 each, and 2^-149 where the result is
+    subnormal), whatever the factors' magnitudes."""
+    rng = np.random.default_rng(2)
+    A = _ones(A0)
+    X = (_mantissas(rng, (A.M, D)) * np.float64(sx)).astype(np.float32)
+    Y = (_mantissas(rng, (A.K, D)) * np.float64(sy)).astype(np.float32)
+    out, want, bound = _sddmm(A, X, Y)
+    assert (np.abs(out - want) <= 68 * (2.0 ** -24 * bound + 2.0 ** -149)).all()
+
+
+def test_sddmm_one_small_element(cuda):
+    """Tiny factors among ordinary ones; blocks of rows with and without them."""
+    rng = np.random.default_rng(3)
+    A = _ones(A0)
+    X, Y = np.zeros((A.M, D), np.float32), _mantissas(rng, (A.K, D))
+    X[:, 5] = _mantissas(rng, A.M)
+    X[40::200, 5] *= np.float32(1e-36)
+    out, want, bound = _sddmm(A, X, Y)
+    assert (np.abs(out - want) <= 1.02 * 2.0 ** -23 * bound + 2.0 ** -149).all()
