@@ -23,6 +23,7 @@
 #include <cudaTypedefs.h>
 
 #include <atomic>
+#include <cfloat>
 #include <mutex>
 
 #include "mma.cuh"
@@ -328,8 +329,8 @@ __global__ void __launch_bounds__(kSpmmCta)
 //
 // The tile product At x B is a dense contraction (32 x win by win x 64 per CTA), and
 // its multiply-adds, two shared loads per 16 of them, were the kernel's time.  Here
-// it runs as mma.m16n8k16 with fp32 accumulation.  A's values are fp32: each is cut
-// exactly into three bf16 parts of 8 bits (x = hi + mid + lo, truncating), so three
+// it runs as mma.m16n8k16 with fp32 accumulation.  A's values are fp32: each is split
+// exactly into three bf16 parts (x = hi + mid + lo, mma.cuh), so three
 // products per step give the exact products x*b that the multiply-add form rounds
 // once; the parts of a step are summed from zero, lowest first, and added to the
 // running sum in fp32.  (tcgen05 needs 64 or 128 rows per tile: a 32-row block's
@@ -341,9 +342,10 @@ __global__ void __launch_bounds__(kSpmmCta)
 // and eight lanes per row then add its off-band nonzeros (16 bytes of B per lane) and
 // store whole lines of C.
 //
-// Splitting an infinity or NaN, or multiplying a zero part by one, would make NaN:
-// a CTA that meets one in its tile or window sums its rows nonzero by nonzero
-// instead.
+// Splitting an infinity or NaN, or multiplying a zero part by one, makes NaN, a value
+// next to the largest splits into infinite parts, and one below 2^-103 has no three
+// parts: a CTA that finds an infinity or NaN among its sums, or such a value in its
+// tile, sums its rows nonzero by nonzero instead.
 //
 // What bounds it now: instructions (58 % of issue slots with 24 warps per SM), most of
 // them in the scatter and the off-band rows; the tensor pipe is 14 % busy.  Measured
@@ -432,7 +434,6 @@ __global__ void __launch_bounds__(kSpmmCta, 6)
   if (t <= kBandRows) rp[t] = __ldg(a.row_ptr + min(i0 + t, M));
   if (t < kBandRows) cnt[t] = 0;
   __syncthreads();
-  float amax = 0.0f;  // the tile's largest magnitude, or NaN
   for (int n0 = 0; n0 < k_end - k_beg; n0 += SQ * kSpmmCta) {
     if (n0 > 0) load(n0);
     int r = 0;  // the last row whose start is <= the thread's first nonzero
@@ -450,7 +451,6 @@ __global__ void __launch_bounds__(kSpmmCta, 6)
           float *cell = at + r * pitch + d;
           const float old = atomicExch(cell, cv[q]);
           if (old != 0.0f) atomicAdd(cell, old);
-          amax = max_nan(amax, cv[q]);
         } else {
           const int slot = atomicAdd(cnt + r, 1);
           if (slot < kBandList) list[r * kBandList + slot] = make_int2(cj[q], __float_as_int(cv[q]));
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kSpmmCta, 6)
   const float *arow = at + (16 * (w & 1) + (lane >> 2)) * pitch + 2 * (lane & 3);
   // B fragments of two n-tiles: lanes 0-15 rows k .. k+15 of columns 8n, 16-31 of 8n + 8
   const uint32_t brow = sm_u32(swz) + (uint32_t)(lane & 15) * 128;
-  uint32_t bmax = 0;  // the window's largest magnitudes (bf16 pairs), or NaN
+  uint32_t least = 0xffffffffu;  // the tile's smallest nonzero magnitude
 #pragma unroll 1
   for (int s = s0; s < s1; ++s) {
     uint32_t hi[4], mid[4], lo[4];
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(kSpmmCta, 6)
     for (int q = 0; q < 4; ++q) {  // a0: row, a1: row + 8, a2, a3: columns + 8
       const float2 v =
           *reinterpret_cast<const float2 *>(arow + (q & 1) * 8 * pitch + 16 * s + (q >> 1) * 8);
-      amax = max_nan(max_nan(amax, v.x), v.y);
+      least = min_nonzero(min_nonzero(least, v.x), v.y);
       split3(v.x, v.y, hi[q], mid[q], lo[q]);
     }
     const uint32_t row = brow + (uint32_t)s * 16 * 128;
@@ -491,8 +491,6 @@ __global__ void __launch_bounds__(kSpmmCta, 6)
     for (int n2 = 0; n2 < 4; ++n2) {
       uint32_t bf[4];
       ldmatrix_x4_trans(bf, row + ((((uint32_t)(2 * n2 + (lane >> 4))) ^ ((row >> 7) & 7)) << 4));
-#pragma unroll
-      for (int q = 0; q < 4; ++q) bmax = max_nan_bf16(bmax, bf[q]);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         float d[4];
@@ -504,9 +502,10 @@ __global__ void __launch_bounds__(kSpmmCta, 6)
       }
     }
   }
-  // An exponent of all ones: infinity or NaN.
-  const bool odd = !(fabsf(amax) <= 3.402823466e38f) || (bmax & 0x7f80u) == 0x7f80u ||
-                   (bmax & 0x7f800000u) == 0x7f800000u;
+  float amax = 0.0f;  // the sums' largest magnitude, or NaN
+#pragma unroll
+  for (int q = 0; q < 32; ++q) amax = max_nan(amax, acc[q / 4][q % 4]);
+  const bool odd = !(fabsf(amax) <= FLT_MAX) || least < kSplitMin;
   const bool direct = __syncthreads_or(odd) != 0;  // the tile and the window are free now
   {
     float *s = sums + (w >> 1) * kBandRows * (kBandCols + kBandCPad) +

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_util import dev
+from gpu_util import dev, to_torch_bf16
 from segtaco_gb300 import native as N
 from segtaco_gb300 import ops, synth
 
@@ -74,3 +74,33 @@ def test_sddmm_one_small_element(cuda):
     X[40::200, 5] *= np.float32(1e-36)
     out, want, bound = _sddmm(A, X, Y)
     assert (np.abs(out - want) <= 1.02 * 2.0 ** -23 * bound + 2.0 ** -149).all()
+
+
+def _spmm(A, B, bf16):
+    cfg = N.Config.make(schedule=N.RB_PR, items_per_unit=32, flags=N.FLAG_WINDOW)
+    Bd = torch.from_numpy(B).cuda()
+    if bf16:
+        bits = synth.to_bf16_bits(B)
+        B, Bd = synth.bf16_bits_to_f32(bits), to_torch_bf16(bits)
+    Ad = dev(A)
+    assert " band " in ops.plan_name(Ad, Bd, cfg)
+    C = ops.spmm(Ad, Bd, torch.full((A.M, B.shape[1]), float("nan"), device="cuda"), cfg).cpu().numpy()
+    rows = np.repeat(np.arange(A.M), np.diff(A.row_ptr))
+    with np.errstate(invalid="ignore"):
+        t = A.val.astype(np.float64)[:, None] * B[A.col].astype(np.float64)
+        want, bound = np.zeros(C.shape), np.zeros(C.shape)
+        np.add.at(want, rows, t)
+        np.add.at(bound, rows, np.abs(t))
+    return C, want, bound
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("sa,sb", [(1e-30, 1.0), (1e-33, 1e10), (1e-36, 1e30), (1e-39, 1e38), (1e-44, 1e38),
+                                   (1.0, 1e-39), (1e-20, 1e-18)])
+def test_spmm_small_magnitudes(cuda, sa, sb, bf16):
+    """Rows of at most 73 nonzeros as near as their multiply-adds, whatever the magnitudes."""
+    rng = np.random.default_rng(4)
+    A = synth.CSR(A0.row_ptr, A0.col, (_mantissas(rng, A0.nnz) * np.float64(sa)).astype(np.float32),
+                  A0.M, A0.K)
+    C, want, bound = _spmm(A, (_mantissas(rng, (A.K, 64)) * np.float64(sb)).astype(np.float32), bf16)
+    assert (np.abs(C - want) <= 73 * (2.0 ** -24 * bound + 2.0 ** -149)).all()
