@@ -130,8 +130,12 @@ __global__ void __launch_bounds__(kSpmmCta, window_min_ctas<BT, V, G>())
 // memory: banded 262,144 rows, N = 64 195 us, now 181; 100,000, N = 128 144, now 133).
 // Off-band nonzeros (outside the window) go to a per-row list of kBandList entries,
 // and each thread gathers its 4 columns of them from global memory, 8 at a time (a
-// row with more walks its nonzeros in global memory instead).  The TMA wait is
-// bounded as in the window kernel (SEGTACO_ETIMEOUT, rows left unwritten).
+// row with more walks its nonzeros in global memory instead).  The tile's zeros make
+// NaN of infinities in the window's unused rows: a thread that ends with an infinity
+// or NaN sums that row again, nonzero by nonzero.  (Five CTAs per SM, what the shared
+// memory allows: 93 registers, banded 262,144 rows, N = 64 183.5 -> 177.8 us against the 79
+// the compiler takes unasked.)  The TMA wait is bounded as in the window kernel
+// (SEGTACO_ETIMEOUT, rows left unwritten).
 constexpr int kBandRows = 32;
 constexpr int kBandCols = 64;
 constexpr int kBandList = 16;
@@ -169,7 +173,7 @@ __host__ __device__ inline BandSmem band_smem(int win) {
   return m;
 }
 
-__global__ void __launch_bounds__(kSpmmCta)
+__global__ void __launch_bounds__(kSpmmCta, 5)
     spmm_band_kernel(SpmmArgs<float> a, const __grid_constant__ CUtensorMap tm, int halo,
                      int *status) {
   const int win = kBandRows + 2 * halo;
@@ -313,6 +317,19 @@ __global__ void __launch_bounds__(kSpmmCta)
           band_fma4(acc[q], ld_val(a.val, k),
                     band_b4(a.B + (size_t)(unsigned)j * a.ldb + c0));
       }
+    }
+  }
+  // An infinity or NaN: from the row's own terms, or from a zero of the tile times an
+  // infinity of the window.  The row again, nonzero by nonzero.
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float amax = max_nan(max_nan(acc[q][0], acc[q][1]), max_nan(acc[q][2], acc[q][3]));
+    if (!(fabsf(amax) <= FLT_MAX)) {
+      acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.0f;
+#pragma unroll 1
+      for (int k = rp[4 * rb + q]; k < rp[4 * rb + q + 1]; ++k)
+        band_fma4(acc[q], ld_val(a.val, k),
+                  band_b4(a.B + (size_t)(unsigned)__ldg(a.col + k) * a.ldb + c0));
     }
   }
 #pragma unroll

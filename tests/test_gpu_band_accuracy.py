@@ -104,3 +104,26 @@ def test_spmm_small_magnitudes(cuda, sa, sb, bf16):
                   A0.M, A0.K)
     C, want, bound = _spmm(A, (_mantissas(rng, (A.K, 64)) * np.float64(sb)).astype(np.float32), bf16)
     assert (np.abs(C - want) <= 73 * (2.0 ** -24 * bound + 2.0 ** -149)).all()
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("n", [64, 80])
+def test_spmm_infinities_of_unused_rows(cuda, n, bf16):
+    """Infinities and NaN of B and A reach the rows that hold them, by the window and off the band, and
+    no others; values near the largest stay finite."""
+    rng = np.random.default_rng(6)
+    keep = np.ones(A0.nnz, bool)
+    keep[np.isin(A0.col, (250, 251, 900))] = False  # unused rows of B
+    rows = np.repeat(np.arange(A0.M), np.diff(A0.row_ptr))
+    ptr = np.append(0, np.cumsum(np.bincount(rows[keep], minlength=A0.M))).astype(np.int32)
+    A = synth.CSR(ptr, A0.col[keep].copy(), _mantissas(rng, int(keep.sum())), A0.M, A0.K)
+    A.val[A.row_ptr[600] + 20], A.val[A.row_ptr[700] + 2] = np.inf, np.nan
+    A.val[A.row_ptr[1300] + 30] = np.float32(3.4e38)
+    B = rng.uniform(0.25, 0.5, (A.K, n)).astype(np.float32)
+    B[250], B[251, ::2], B[900, 1::3] = np.inf, np.nan, -np.inf
+    B[1000, 7], B[1100, 9] = np.inf, np.nan
+    C, want, bound = _spmm(A, B, bf16)
+    finite = np.isfinite(want)
+    assert finite.mean() > 0.9
+    assert np.array_equal(C[~finite], want[~finite].astype(np.float32), equal_nan=True)
+    assert (np.abs(C - want)[finite] <= 73 * 2.0 ** -24 * bound[finite]).all()
