@@ -721,6 +721,26 @@ static bool holds_sums(const SpmmPlan &plan, const void *workspace, size_t bytes
   return bytes >= plan.workspace && ((uintptr_t)workspace & 255) == 0;
 }
 
+// Whether segtaco_spmm_partition, which knows neither B nor its pitch, made what `plan`
+// reads from this workspace.  Another alignment or pitch of B can change the lanes, and
+// with them the pieces' layout or the chunks' size, and a row pitch from 4 GB takes
+// pieces where the partition had joined chunks in mind and prepared nothing.
+static bool partition_serves(const SpmmPlan &plan, int M, int K, long long nnz, int N, int b_dtype,
+                             const float *C, long long ldc, const segtaco_config *cfg,
+                             const void *workspace, size_t bytes) {
+  SpmmPlan p;
+  if (plan_spmm(M, K, nnz, N, b_dtype, N, ldc, nullptr, C, cfg, &p) != SEGTACO_OK) return false;
+  if (p.walk == kWalkSplitJoin && !holds_sums(p, workspace, bytes) &&
+      plan_spmm(M, K, nnz, N, b_dtype, N, ldc, nullptr, C, cfg, &p, LongRowScratch::kPieces) !=
+          SEGTACO_OK)
+    return false;
+  const bool pieces = plan.piece_len > 0;
+  return p.px_entries == plan.px_entries && p.py_entries == plan.py_entries &&
+         p.items_per_unit == plan.items_per_unit && p.long_row == plan.long_row &&
+         p.piece_len == plan.piece_len && p.piece_parts == plan.piece_parts &&
+         (!pieces || (p.slabs == plan.slabs && p.W == plan.W));
+}
+
 int segtaco_spmm(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr, const int32_t *col,
                  const float *vals, const void *B, int32_t b_dtype, int64_t ldb, float *C,
                  int64_t ldc, int32_t N, const segtaco_config *cfg, void *workspace,
@@ -740,7 +760,9 @@ int segtaco_spmm(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr, cons
     SEGTACO_TRY(plan_spmm(M, K, nnz, N, b_dtype, ldb, ldc, B, C, cfg, &plan,
                           LongRowScratch::kPieces));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const bool ready = cfg && (cfg->flags & SEGTACO_FLAG_PARTITION_READY);
+  bool ready = cfg && (cfg->flags & SEGTACO_FLAG_PARTITION_READY);
+  if (ready && workspace && plan.workspace)
+    ready = partition_serves(plan, M, K, nnz, N, b_dtype, C, ldc, cfg, workspace, workspace_bytes);
   const bool search = !ready && plan.walk == kWalkSplit && (long long)M * N <= kSearchMaxElems;
   Scratch scratch(workspace, workspace_bytes, s);
   if (workspace || !search)  // (a caller's workspace is checked, if not needed)
