@@ -981,7 +981,7 @@ int segtaco_spmspv(int32_t M, int32_t K, int64_t nnz, const int32_t *col_ptr,
   if (nx < 0) return set_error(SEGTACO_EINVAL, "negative nx");
   if (M > 0 && y == nullptr) return set_error(SEGTACO_EINVAL, "y is NULL");
   if (nx > 0 && (!x_idx || !x_vals)) return set_error(SEGTACO_EINVAL, "x is NULL");
-  return launch_spmspv(M, K, col_ptr, row_idx, vals, nx, x_idx, x_vals, y,
+  return launch_spmspv(M, K, nnz, col_ptr, row_idx, vals, nx, x_idx, x_vals, y,
                        static_cast<cudaStream_t>(stream));
 }
 

@@ -321,7 +321,8 @@ int device_sms();
 
 int launch_spmv(int M, long long nnz, const int *row_ptr, const int *col, const float *val,
                 const float *x, float *y, cudaStream_t s);
-int launch_spmspv(int M, int K, const int *col_ptr, const int *row_idx, const float *val, int nx,
-                  const int *x_idx, const float *x_vals, float *y, cudaStream_t s);
+int launch_spmspv(int M, int K, long long nnz, const int *col_ptr, const int *row_idx,
+                  const float *val, int nx, const int *x_idx, const float *x_vals, float *y,
+                  cudaStream_t s);
 
 }  // namespace segtaco
