@@ -418,12 +418,7 @@ int plan_batch_problem(const segtaco_spmm_problem &p, const segtaco_config *cfg,
   c.flags &= ~(SEGTACO_FLAG_SMEM_RING | SEGTACO_FLAG_TMA_BULK | SEGTACO_FLAG_PARTITION_READY);
   // The persistent kernel walks every row of its items (no long-row CTAs).
   c.flags &= ~SEGTACO_FLAG_LONG_ROWS;
-  segtaco_config planned = c;  // row blocks: the row walk
-  if ((c.schedule == SEGTACO_RB_SR || c.schedule == SEGTACO_RB_PR) &&
-      !(c.flags & SEGTACO_FLAG_FLAT_WALK))
-    planned.flags |= SEGTACO_FLAG_ROW_WALK;
-  SEGTACO_TRY(
-      plan_spmm(p.M, p.K, p.nnz, p.N, p.b_dtype, p.ldb, p.ldc, p.B, p.C, &planned, plan));
+  SEGTACO_TRY(plan_spmm(p.M, p.K, p.nnz, p.N, p.b_dtype, p.ldb, p.ldc, p.B, p.C, &c, plan));
   // The persistent kernel hides the row walk's round trips behind other problems'
   // items, so the split walk pays there where it saves passes over A or narrow
   // loads: slabs of more than 64 columns, and operands without 16-byte lanes, over
@@ -434,19 +429,23 @@ int plan_batch_problem(const segtaco_spmm_problem &p, const segtaco_config *cfg,
   // products are all that small end on a nearly empty split group (16 problems, three
   // wide ones of up to 257,000 items: 136 us against 146), and beside larger ones they
   // cost the same either way (24 problems 434 / 450, 48 problems 395 / 395).
-  if (plan->walk == kWalkSplit && !cfg) {
+  // A caller's configuration: the row walk for fp32 eb_pr on slabs of up to 64 columns alone
+  // (the 48 products of one N, each tuned by itself, split walk / row walk: N = 16 398 / 356
+  // us, 32 494 / 455, 64 685 / 601; bf16 and eb_sr are the faster by the split walk: N = 64
+  // bf16 575 / 608, eb_sr 570 / 708).
+  // The configuration as stored makes this plan again.
+  if (plan->walk == kWalkSplit) {
     const int esz = p.b_dtype == SEGTACO_BF16 ? 2 : 4;
-    if (plan->split_elems * esz == 16 &&
-        (plan->W <= 64 || (long long)p.M + p.nnz < 300000)) {
+    const bool row_walk =
+        cfg ? esz == 4 && c.schedule == SEGTACO_EB_PR && plan->W <= 64
+            : plan->W <= 64 || (long long)p.M + p.nnz < 300000;
+    if (plan->split_elems * esz == 16 && row_walk) {
       if (c.col_tile <= 0) c.col_tile = std::min(p.N, 256 / esz);
-      segtaco_config rows = c;
-      rows.flags |= SEGTACO_FLAG_ROW_WALK;
-      SEGTACO_TRY(
-          plan_spmm(p.M, p.K, p.nnz, p.N, p.b_dtype, p.ldb, p.ldc, p.B, p.C, &rows, plan));
-    } else if (c.items_per_unit > 128) {
+      c.flags |= SEGTACO_FLAG_ROW_WALK;
+    } else if (!cfg && c.items_per_unit > 128) {
       c.items_per_unit = 128;
-      SEGTACO_TRY(plan_spmm(p.M, p.K, p.nnz, p.N, p.b_dtype, p.ldb, p.ldc, p.B, p.C, &c, plan));
     }
+    SEGTACO_TRY(plan_spmm(p.M, p.K, p.nnz, p.N, p.b_dtype, p.ldb, p.ldc, p.B, p.C, &c, plan));
   }
   *used = c;
   return SEGTACO_OK;
