@@ -116,8 +116,11 @@ __global__ void __launch_bounds__(kSpmmCta, spmm_min_ctas<V, G, false>())
 // staged in dynamic shared memory after the problems' item_begin values, and the
 // next item drawn while the current one is walked (the draw is a round trip to L2).
 // `D`: the largest chunk of the group's problems.
+// Warps per SM: 32, 28 for 8 bf16 elements; at 36 and 32 the item loop spills (the pool's 48
+// products of one N, 36 / 32 / 28 warps: fp32 N = 128 886 / 852 / 871 us, N = 37 532 / 531 /
+// 573; bf16 N = 128, 32 and 28 790 / 745).
 template <typename BT, int E, int C, int G>
-__global__ void __launch_bounds__(kSpmmCta, split_min_ctas<BT, E, C, G>())
+__global__ void __launch_bounds__(kSpmmCta, E > 4 ? 7 : 8)
     spmm_batch_split_kernel(const BatchProblem<BT> *__restrict__ probs,
                             const long long *__restrict__ item_begin, int nprobs,
                             long long total_items, unsigned long long *__restrict__ queue,
