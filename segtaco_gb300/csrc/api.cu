@@ -640,7 +640,10 @@ int segtaco_autotune_heuristic(int32_t M, int32_t K, int64_t nnz, int32_t N, int
     while (cfg->rows_per_unit > 1 && M / cfg->rows_per_unit < 8192) cfg->rows_per_unit >>= 1;
   // rb: 8 loads in flight in the row walk, or (4) even rows side by side.
   // (rb_pr's rows of more than 32 nonzeros in 16-byte lanes stay with the row walk;
-  // 8 with long rows would ask for joined chunks, even rows keep the pieces.)
+  // 8 with long rows would ask for joined chunks, even rows keep the pieces.  Even rows
+  // of rb_sr that fill the lanes, fp32 beyond 64 columns, get the row walk with 4 loads: 8
+  // / 4 loads, rows of 16, N = 96 and 128, 16,384 10.8 / 10.2 and 11.0 / 10.7 us, 100,000
+  // 50.7 / 49.7 and 54.7 / 54.7; 100,000 banded rows of 73 175 / 168 and 179 / 168.)
   const bool side_by_side =
       even &&
       (schedule == SEGTACO_RB_SR || nnz <= 32LL * M || N % (16 / esz) != 0 || long_rows);
