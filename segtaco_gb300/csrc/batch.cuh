@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kSpmmCta, spmm_min_ctas<V, G, false>())
 // `D`: the largest chunk of the group's problems.
 // Warps per SM: 32, 28 for 8 bf16 elements; at 36 and 32 the item loop spills (the pool's 48
 // products of one N, 36 / 32 / 28 warps: fp32 N = 128 886 / 852 / 871 us, N = 37 532 / 531 /
-// 573; bf16 N = 128, 32 and 28 790 / 745).
+// 573; bf16 N = 128, 32 and 28 763 / 721).
 template <typename BT, int E, int C, int G>
 __global__ void __launch_bounds__(kSpmmCta, E > 4 ? 7 : 8)
     spmm_batch_split_kernel(const BatchProblem<BT> *__restrict__ probs,

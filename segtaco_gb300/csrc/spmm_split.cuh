@@ -106,6 +106,11 @@ __device__ __forceinline__ ChunkEdges search_edges(const SpmmArgs<BT> &a, long l
 // JOIN (rb_pr, spmm_join.cu): chunk w's sums of rows cut by its edges are stored in
 // a.piece_part -- two rows of a.piece_ld floats, the row it starts in, then the row
 // open at its end -- instead of being added to C.
+// Steps in which some row ends sum their terms by themselves too, but for 8 bf16 elements
+// per lane: their registers cost warps or spill, and the gathers' round trips need the
+// warps (bf16, N = 128, 36 warps without / 32 with: 400,000 lognormal rows 158 / 187 us,
+// 200,000 80 / 97).  Error against FP64, one chain per row / all but those steps / all, bf16,
+// N = 64: lognormal rows 8.5e-8 / 7.9e-8 / 6.4e-8, power-law 1.8e-7 / 1.5e-7 / 1.4e-7.
 template <typename BT, int E, int C, int G, bool JOIN = false>
 __device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, const ChunkEdges ce,
                                                 int slab, int lane, int D,
@@ -113,6 +118,7 @@ __device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, const Chu
   constexpr int P = 32 / G;
   constexpr int V = E * C;
   constexpr int S = kSplitStep;
+  constexpr bool kStepSums = E <= 4;
   using Dn = Dense<BT, E>;
   const unsigned FULL = 0xffffffffu;
   int *cs = sm;
@@ -239,31 +245,41 @@ __device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, const Chu
     }
     const float4 v4 = *reinterpret_cast<const float4 *>(vs + q);
     const float vv[S] = {v4.x, v4.y, v4.z, v4.w};
-    float part[V];  // the step's terms of the open row
+    // The step's terms of the open row, or (kStepSums false) the row's sum itself.
+    float terms[kStepSums ? V : 1];
+    float *part = kStepSums ? terms : acc;
     auto add = [&](int u, bool begin) {
 #pragma unroll
       for (int c = 0; c < C; ++c)
 #pragma unroll
         for (int e = 0; e < E; ++e) {
           const float x = Dn::get(b[u][c], e);
-          part[c * E + e] = begin ? vv[u] * x : fmaf(vv[u], x, part[c * E + e]);
+          part[c * E + e] = kStepSums && begin ? vv[u] * x : fmaf(vv[u], x, part[c * E + e]);
         }
     };
     auto close = [&]() {
+      if constexpr (kStepSums) {
 #pragma unroll
-      for (int v = 0; v < V; ++v) acc[v] += part[v];
+        for (int v = 0; v < V; ++v) acc[v] += terms[v];
+      }
+    };
+    auto clear = [&]() {
+      if constexpr (kStepSums) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) terms[v] = 0.0f;
+      }
     };
     const int p = ybase + q;
     if (t == steps || (t == 0 && ragged0) || (t == steps - 1 && ragged1)) {
       // positions outside the chunk, or runs that have ended
-      zero<V>(part);
+      clear();
 #pragma unroll
       for (int u = 0; u < S; ++u) {
         if (p + u >= lo && p + u < hi) {
           if (p + u == rend) {
             close();
             next_row(p + u);
-            zero<V>(part);
+            clear();
           }
           add(u, false);
         }
@@ -286,7 +302,7 @@ __device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, const Chu
           if (p + u == rend) {
             if (u > 0) close();
             next_row(p + u);
-            if (u > 0) zero<V>(part);
+            if (u > 0) clear();
           }
           __syncwarp();
         }
@@ -327,11 +343,9 @@ __device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, const Chu
   }
 }
 
-// Warps per SM: 36 at 56 registers, 32 at 64 for several chunks per lane and for 8 bf16
-// elements (250,000 power-law rows, bf16, 36 warps / 32: N = 64 98 / 86 us, N = 128 164 /
-// 153; 90,000 rows of 16, N = 128 49 / 41).
+// Warps per SM: 36 at 56 registers, 32 at 64 for several chunks per lane.
 template <typename BT, int E, int C, int G> constexpr int split_min_ctas() {
-  return (C > 1 || E > 4 ? 32 : 36) / kSpmmWarps;
+  return (C > 1 ? 32 : 36) / kSpmmWarps;
 }
 
 // a.part_x null: the chunk's edges are searched here (and, but for JOIN, C is zero on
