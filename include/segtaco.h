@@ -50,7 +50,9 @@ extern "C" {
 #define SEGTACO_RB_SR 0 /* row-balanced, sequential reduction     (spmm_rb_sr.h) */
 #define SEGTACO_RB_PR 1 /* row-balanced, parallel reduction       (spmm_rb_pr.h) */
 #define SEGTACO_EB_SR 2 /* element-balanced, sequential reduction (spmm_eb_sr.h) */
-#define SEGTACO_EB_PR 3 /* element-balanced, parallel reduction   (spmm_eb_pr.h) */
+#define SEGTACO_EB_PR 3 /* element-balanced, parallel reduction   (spmm_eb_pr.h);
+                           by default both walk equal chunks in the same order: runs
+                           of a row's nonzeros summed side by side, then together  */
 
 /* ---- dense operand types ------------------------------------------------ */
 #define SEGTACO_F32 0
@@ -135,12 +137,17 @@ typedef struct segtaco_config {
                              result does not vary from run to run          */
   uint32_t flags;         /* SEGTACO_FLAG_*                                        */
   int32_t depth;          /* row walk: dense loads in flight per lane (0 = 4, 4, 8);  */
-                          /* 4 with a row-block schedule: rows are even, several of  */
-                          /* a block are walked side by side; 8 with rb_pr and       */
-                          /* SEGTACO_FLAG_LONG_ROWS: rows are uneven, equal chunks   */
-                          /* of the matrix are walked and the rows they cut summed   */
-                          /* in order (any nnz; not with fp32 vec 8 or k_parts > 1;  */
-                          /* where the workspace holds the sums)                     */
+                          /* 4 with a row-block schedule also says that rows are     */
+                          /* even: several of a block are walked side by side and    */
+                          /* rows_per_unit does not count (0, or 4 with ROW_WALK:    */
+                          /* four loads, whatever the rows); 8 with rb_pr and        */
+                          /* SEGTACO_FLAG_LONG_ROWS says that they are uneven: equal */
+                          /* chunks of the matrix are walked and the rows they cut   */
+                          /* summed in order, in a workspace of two rows of C per    */
+                          /* chunk, and rows_per_unit does not count.  Any nnz, but  */
+                          /* from 1M on only with items_per_unit 0 or 512; not with  */
+                          /* ROW_WALK, fp32 vec 8 or k_parts > 1, nor where the      */
+                          /* workspace does not hold the sums: pieces                */
   int32_t k_parts;        /* rb_pr pieces: passes over ranges of B's rows, 1 .. 8
                              (0: one).  With more than one the pieces (of
                              2048 nonzeros) run in a launch of their own

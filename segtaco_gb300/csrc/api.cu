@@ -173,6 +173,16 @@ static bool split_shape(const segtaco_config &c, int N, int K, int esz, F fits, 
   return true;
 }
 
+// Whether a configuration asks for rb_pr's joined chunks (spmm_join.cu): depth 8 with
+// SEGTACO_FLAG_LONG_ROWS, and from 1M nonzeros on the default threshold (another one asks
+// for pieces of the rows it names).
+static bool asks_join(const segtaco_config &c, long long nnz) {
+  return c.schedule == SEGTACO_RB_PR && nnz > 0 && c.depth == 8 && c.k_parts <= 1 &&
+         (c.flags & SEGTACO_FLAG_LONG_ROWS) &&
+         !(c.flags & (SEGTACO_FLAG_ROW_WALK | SEGTACO_FLAG_FLAT_WALK)) &&
+         (nnz < kLongRowsMinNnz || c.items_per_unit <= 0 || c.items_per_unit == kPieceThreshold);
+}
+
 int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, long long ldc,
               const void *B, const float *C, const segtaco_config *cfg, SpmmPlan *plan,
               LongRowScratch scratch) {
@@ -180,6 +190,13 @@ int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, lo
   c.schedule = SEGTACO_AUTO;
   if (cfg) c = *cfg;
   const int esz = b_dtype == SEGTACO_BF16 ? 2 : 4;
+  // A configuration for joined chunks (below) planned without them: over a B beyond L2
+  // the lanes that segtaco_autotune_heuristic chooses for pieces.  Measured on GB300,
+  // segtaco_spmm_noalloc, lognormal rows, fp32, 16-byte / 32-byte lanes: 400,000, N = 64
+  // 244 / 208 us, 128 526 / 474; 100,000, N = 128 125 / 111.
+  if (scratch != LongRowScratch::kJoin && asks_join(c, nnz) && c.vec == 0 && c.col_tile == 0 &&
+      (double)K * N * esz > 48e6 && N % (32 / esz) == 0)
+    c.vec = 32 / esz;
   // Vector width: the widest 16-byte-or-less load that N, the strides and the
   // base pointers allow, for both the B loads and the C stores.
   // fp32 also takes vec = 8 on request: one 32-byte load per lane.
@@ -386,23 +403,25 @@ int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, lo
       plan->nchunks = (M + rows - 1) / rows;
     }
   }
-  // rb_pr over rows known to be uneven (depth 8 with SEGTACO_FLAG_LONG_ROWS, which
-  // segtaco_autotune_heuristic sets for them): merge-path chunks whose sums of cut
-  // rows are added in order (spmm_join.cu) instead of pieces and row blocks.  fp32's
-  // explicit 32-byte lanes (split_shape) and passes over B keep the pieces.
-  if (schedule == SEGTACO_RB_PR && scratch == LongRowScratch::kJoin && nnz > 0 && c.depth == 8 &&
-      c.k_parts <= 1 && (c.flags & SEGTACO_FLAG_LONG_ROWS) && !plan->use_tma &&
-      plan->band_halo < 0 && plan->window_halo < 0 &&
-      !(c.flags & (SEGTACO_FLAG_ROW_WALK | SEGTACO_FLAG_FLAT_WALK)) &&
-      ldb * esz < (1LL << 32) && ldc * 4 < (1LL << 32)) {
-    if (split_shape(c, N, K, esz, fits, plan)) {
-      plan->walk = kWalkSplitJoin;
-      plan->long_row = plan->piece_len = 0;
-      plan->piece_parts = 1;
-      plan->items_per_unit = default_chunk_items(M, nnz);
-      plan->nchunks = (M + nnz + plan->items_per_unit - 1) / plan->items_per_unit;
-      plan->px_entries = 2 * plan->nchunks * (((long long)N + 3) & ~3LL);
-      plan->py_entries = 0;
+  // rb_pr over rows known to be uneven (asks_join, as segtaco_autotune_heuristic sets for
+  // them): merge-path chunks whose sums of cut rows are added in order (spmm_join.cu)
+  // instead of pieces and row blocks.  fp32's explicit 32-byte lanes (split_shape) and
+  // passes over B keep the pieces.
+  if (scratch == LongRowScratch::kJoin && asks_join(c, nnz) && !plan->use_tma &&
+      plan->band_halo < 0 && plan->window_halo < 0) {
+    SpmmPlan t = *plan;
+    if (split_shape(c, N, K, esz, fits, &t)) {
+      t.walk = kWalkSplitJoin;
+      t.long_row = t.piece_len = 0;
+      t.piece_parts = 1;
+      t.items_per_unit = default_chunk_items(M, nnz);
+      t.nchunks = (M + nnz + t.items_per_unit - 1) / t.items_per_unit;
+      t.px_entries = 2 * t.nchunks * (((long long)N + 3) & ~3LL);
+      t.py_entries = 0;
+      if (ldb * esz >= (1LL << 32) || ldc * 4 >= (1LL << 32))
+        return plan_spmm(M, K, nnz, N, b_dtype, ldb, ldc, B, C, cfg, plan,
+                         LongRowScratch::kPieces);
+      *plan = t;
     }
   }
   if (plan->px_entries)
@@ -627,7 +646,14 @@ int segtaco_autotune_heuristic(int32_t M, int32_t K, int64_t nnz, int32_t N, int
   // with B in L2 (banded, N = 64) 8 stays faster (0.224 vs 0.235 ms).
   if (!sequential && esz == 2 && bbytes > 48e6 && N % 16 == 0 && (skewed || nnz >= 4000000))
     cfg->vec = 16;
-  if (split || join) cfg->col_tile = cfg->vec = 0;
+  // (joined chunks: a slab for the pieces that may take their place, where it covers N and
+  // so changes nothing for the chunks.  segtaco_spmm_noalloc, 100,000 lognormal rows, 32
+  // fp32 / 64 bf16 columns against 64 / 128: N = 64 fp32 65 / 55 us, N = 128 bf16 88 / 70;
+  // 60,000 power-law rows, N = 64 67 / 108.)
+  const bool piece_tile = join && !((double)max_row_len > 256.0 * mean) && N <= 256 / esz &&
+                          bbytes <= 48e6;
+  if (split || join) cfg->vec = 0;
+  if (split || join) cfg->col_tile = piece_tile ? 256 / esz : 0;
   // eb: merge-path items per chunk; rb: the long-row threshold.
   cfg->items_per_unit = (schedule == SEGTACO_RB_SR || schedule == SEGTACO_RB_PR)
                             ? (int)kLongRowDefault
