@@ -146,8 +146,9 @@ typedef struct segtaco_config {
                           /* summed in order, in a workspace of two rows of C per    */
                           /* chunk, and rows_per_unit does not count.  Any nnz, but  */
                           /* from 1M on only with items_per_unit 0 or 512; not with  */
-                          /* ROW_WALK, fp32 vec 8 or k_parts > 1, nor where the      */
-                          /* workspace does not hold the sums: pieces                */
+                          /* ROW_WALK, fp32 vec 8 or k_parts > 1, nor where the sums */
+                          /* would pass 64 MB for rows of more than 32 nonzeros and  */
+                          /* N <= 256, or the workspace does not hold them: pieces   */
   int32_t k_parts;        /* rb_pr pieces: passes over ranges of B's rows, 1 .. 8
                              (0: one).  With more than one the pieces (of
                              2048 nonzeros) run in a launch of their own

@@ -182,6 +182,15 @@ static bool asks_join(const segtaco_config &c, long long nnz) {
          !(c.flags & (SEGTACO_FLAG_ROW_WALK | SEGTACO_FLAG_FLAT_WALK)) &&
          (nnz < kLongRowsMinNnz || c.items_per_unit <= 0 || c.items_per_unit == kPieceThreshold);
 }
+// Where the sums of joined chunks (two rows of C per chunk of up to 512 items) outgrow the
+// scratch kept between calls and C's own traffic, the pieces are the faster: rows of 500
+// nonzeros, 233,000, N = 128 3.77 ms joined and waited for, 3.12 in pieces (with a workspace
+// 3.33 / 3.10); of 1500, 50,000, N = 64 and 256 1.24 / 1.03 and 4.72 / 3.94; of 100, 200,000,
+// N = 256 1.38 / 1.31.  Not beyond 256 columns, where the pieces walk A for each 32 of
+// them (rows of 500, N = 512 15.3 / 25.7), nor for rows of 20 (400,000, N = 512 1.39 / 2.11).
+static bool sums_too_large(int M, long long nnz, int N, double bytes) {
+  return nnz >= kLongRowsMinNnz && N <= 256 && nnz > 32LL * M && bytes > (double)kScratchKeep;
+}
 
 int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, long long ldc,
               const void *B, const float *C, const segtaco_config *cfg, SpmmPlan *plan,
@@ -418,7 +427,8 @@ int plan_spmm(int M, int K, long long nnz, int N, int b_dtype, long long ldb, lo
       t.nchunks = (M + nnz + t.items_per_unit - 1) / t.items_per_unit;
       t.px_entries = 2 * t.nchunks * (((long long)N + 3) & ~3LL);
       t.py_entries = 0;
-      if (ldb * esz >= (1LL << 32) || ldc * 4 >= (1LL << 32))
+      if (ldb * esz >= (1LL << 32) || ldc * 4 >= (1LL << 32) ||
+          sums_too_large(M, nnz, N, t.px_entries * 4.0))
         return plan_spmm(M, K, nnz, N, b_dtype, ldb, ldc, B, C, cfg, plan,
                          LongRowScratch::kPieces);
       *plan = t;

@@ -48,3 +48,27 @@ def test_b_without_16_byte_rows(cuda, cfg):
     Bd = torch.from_numpy(B).cuda()[:, 1:]
     host = np.ascontiguousarray(B[:, 1:])
     assert_spmm_close(_prepared(A, Bd, **dict(cfg)), A, host, ref=spmm_ref(A, host))
+
+
+@pytest.mark.parametrize("n", [40, 64, 200])
+def test_large_sums_run_as_pieces(cuda, n):
+    """Rows of 100 nonzeros and more whose joined sums would pass 64 MB: the size query, the partition and
+    the product agree on the pieces (n = 200); below, on joined chunks."""
+    rng = np.random.default_rng(n)
+    lens = np.minimum(rng.lognormal(np.log(450.0) - 0.5, 1.0, 50_000).astype(np.int64), 20_000)
+    ptr = np.r_[0, np.cumsum(lens)].astype(np.int32)
+    K = 2000
+    A = synth.CSR(ptr, rng.integers(0, K, int(ptr[-1])).astype(np.int32),
+                  rng.uniform(-1, 1, int(ptr[-1])).astype(np.float32), len(lens), K)
+    B = synth.dense(K, n, seed=n)
+    Ad, Bd = dev(A), torch.from_numpy(B).cuda()
+    cfg = N.Config.make(schedule="rb_pr", depth=8, flags=LR)
+    assert ops.plan_name(Ad, Bd, cfg).startswith("rb_pr pieces ") == (n == 200)
+    ref = spmm_ref(A, B)
+    want = ops.spmm(Ad, Bd, None, cfg)
+    assert_spmm_close(want.cpu().numpy(), A, B, ref=ref)
+    ws = torch.full((ops.spmm_workspace_size(Ad, n, N.F32, cfg),), 0xff, dtype=torch.uint8, device="cuda")
+    C = torch.full((A.M, n), float("nan"), device="cuda")
+    ops.spmm_partition(Ad, C, cfg, ws)
+    ops.spmm(Ad, Bd, C, N.Config.make(schedule="rb_pr", depth=8, flags=LR | READY), ws)
+    assert torch.equal(C, want)

@@ -57,3 +57,16 @@ def test_the_pieces_slab_leaves_the_chunks_as_they_are(native_lib, dtype, n):
     bare = N.Config.make(schedule="rb_pr", depth=8, flags=LR)
     a, b = plan(L, M, 24 * M, n, dtype, c), plan(L, M, 24 * M, n, dtype, bare)
     assert " walk=7 " in a and a.split(" rows_per_unit")[0] == b.split(" rows_per_unit")[0]
+
+
+def test_large_sums_give_way_to_pieces(native_lib):
+    """Two rows of N sums per chunk are no more than 64 MB where rows are long and N <= 256."""
+    L = native_lib
+    c = N.Config.make(schedule="rb_pr", depth=8, flags=LR)
+    for M, mean, n, joined in ((233_000, 500, 128, False), (50_000, 1500, 64, False), (200_000, 100, 256, False),
+                               (200_000, 100, 128, True), (233_000, 500, 512, True), (400_000, 20, 256, True)):
+        name = plan(L, M, M * mean, n, N.F32, c, K=200_000)
+        assert (" walk=7 " in name) == joined, name
+        ws = workspace(L, M, M * mean, n, N.F32, c, K=200_000)
+        if not joined:
+            assert name.startswith("rb_pr pieces ") and ws < 64 << 20
