@@ -989,6 +989,7 @@ int segtaco_sddmm_ex(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr,
     return launch_sddmm_band(M, K, nnz, row_ptr, col, vals, X, Y, x_dtype, ldx, ldy, D, out, s);
   if (c.kernel == SEGTACO_SDDMM_BAND) c.kernel = SEGTACO_SDDMM_AUTO;
   const long long nblk = (nnz + P - 1) / P;
+  const bool x_first = sddmm_x_first(M, K, D, x_dtype);
   if (c.kernel == SEGTACO_SDDMM_AUTO && c.lanes == 0 && sddmm_gather_applies(x_dtype, ldx, ldy)) {
     // Dot products of 512 bytes and more in 32-byte lanes stay with the fixed-shape
     // kernel, two loads per lane (banded, 100,000 rows, D = 128 fp32: 219 us against
@@ -996,14 +997,15 @@ int segtaco_sddmm_ex(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr,
     const SddmmShape sh = sddmm_shape(x_dtype, D, ldx, ldy, X, Y, 0);
     if ((sh.family == 1 || sh.family == 2) && sh.KI == 2 && sh.G >= 8)
       return launch_sddmm(M, nnz, row_ptr, col, vals, X, Y, x_dtype, ldx, ldy, D, out, nullptr,
-                          (int)P, nblk, s, false, 0, SEGTACO_SDDMM_FIXED);
-    return launch_sddmm_gather(M, nnz, row_ptr, col, vals, X, Y, x_dtype, ldx, ldy, D, out, (int)P, s);
+                          (int)P, nblk, s, false, 0, SEGTACO_SDDMM_FIXED, x_first);
+    return launch_sddmm_gather(M, nnz, row_ptr, col, vals, X, Y, x_dtype, ldx, ldy, D, out, (int)P,
+                               x_first, s);
   }
   Scratch scratch(nullptr, 0, s);
   SEGTACO_TRY(scratch.reserve(align256((size_t)(nblk + 1) * sizeof(int))));
   int *starts = static_cast<int *>(scratch.take((nblk + 1) * sizeof(int)));
   return launch_sddmm(M, nnz, row_ptr, col, vals, X, Y, x_dtype, ldx, ldy, D, out, starts, (int)P,
-                      nblk, s, false, c.lanes, c.kernel);
+                      nblk, s, false, c.lanes, c.kernel, x_first);
 }
 
 int segtaco_sddmm(int32_t M, int32_t K, int64_t nnz, const int32_t *row_ptr, const int32_t *col,

@@ -219,12 +219,14 @@ int launch_sddmm_band(int M, int K, long long nnz, const int *row_ptr, const int
 bool sddmm_gather_applies(int x_dtype, long long ldx, long long ldy);
 int launch_sddmm_gather(int M, long long nnz, const int *row_ptr, const int *col,
                         const float *val, const void *X, const void *Y, int x_dtype,
-                        long long ldx, long long ldy, int D, float *out, int P, cudaStream_t s);
+                        long long ldx, long long ldy, int D, float *out, int P, bool x_first,
+                        cudaStream_t s);
+// Whether X's rows should leave L2 first (`x_first`).
+bool sddmm_x_first(int M, int K, int D, int x_dtype);
 int launch_sddmm(int M, long long nnz, const int *row_ptr, const int *col, const float *val,
                  const void *X, const void *Y, int x_dtype, long long ldx, long long ldy, int D,
                  float *out, int *starts, int P, long long nblk, cudaStream_t s,
-                 bool starts_ready = false, int lanes = 0,
-                 int kernel = 0);
+                 bool starts_ready = false, int lanes = 0, int kernel = 0, bool x_first = false);
 // ---- long rows of the row-block schedules (spmm_long.cu) ----
 // Row-block products below this many nonzeros walk every row in the row-block
 // kernel: the list pass and the fork would cost more than a long row there.

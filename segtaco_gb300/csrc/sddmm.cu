@@ -119,12 +119,11 @@ __global__ void __launch_bounds__(kCta, 3) sddmm_kernel(int M, long long nnz,
   }
 }
 
-// A row of X is read once, or for skewed rows by neighbouring warps: it leaves L2 to Y's
-// rows, as the results do.  Measured on GB300, X evict-normal / evict-first: 300,000
-// power-law rows, D = 128 bf16 187 / 184 us, D = 64 fp32 167 / 162; 200,000 rows of 16, D =
-// 128 fp32 155 / 150; where X and Y stay in L2 from call to call it costs up to 10 %
-// (90,862 rows of 16, D = 32 bf16 18.2 / 20.0), and a choice in the kernel costs the gain.
-__device__ __forceinline__ uint64_t sddmm_policy_x() { return l2_policy_evict_first(); }
+// A row of X is read once, or for skewed rows by neighbouring warps: where X and Y do not
+// stay in L2 from call to call, it leaves L2 to Y's rows (the results are streamed).
+__device__ __forceinline__ uint64_t sddmm_policy_x(bool first) {
+  return first ? l2_policy_evict_first() : l2_policy_evict_normal();
+}
 
 // The default kernel.  G lanes hold one dot product, each lane C chunks of E
 // elements (32 bytes where D, ldx, ldy and the pointers allow it, else 16, else one
@@ -153,7 +152,8 @@ template <typename XT, int E, int C, int G, bool FULL>
 __global__ void __launch_bounds__(kCta, 4) sddmm_gather_kernel(
     int M, unsigned nnz, const int *__restrict__ row_ptr, const int *__restrict__ col,
     const float *__restrict__ val, const XT *__restrict__ X, const XT *__restrict__ Y,
-    unsigned ldx, unsigned ldy, int D, float *__restrict__ out, unsigned nblk, unsigned blk) {
+    unsigned ldx, unsigned ldy, int D, float *__restrict__ out, unsigned nblk, unsigned blk,
+    bool x_first) {
   constexpr int P = 32 / G;
   constexpr int U = sddmm_steps<E * (int)sizeof(XT), G>();
   using Dv = Dense<XT, E>;
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kCta, 4) sddmm_gather_kernel(
   const unsigned w = blockIdx.x * (kCta / 32) + threadIdx.x / 32;
   if (w >= nblk) return;  // whole warp leaves together
   const uint64_t pol = l2_policy_evict_normal();
-  const uint64_t polx = sddmm_policy_x();
+  const uint64_t polx = sddmm_policy_x(x_first);
   const unsigned pb = w * blk;
   const unsigned pe = nnz - pb < blk ? nnz : pb + blk;
   auto load_cols = [&](unsigned p) { return p + lane < pe ? ld_stream(col + (p + lane)) : 0; };
@@ -311,14 +311,14 @@ __device__ __forceinline__ void sddmm_fixed_block(
     int M, long long nnz, const int *__restrict__ row_ptr, const int *__restrict__ col,
     const float *__restrict__ val, const XT *__restrict__ X, const XT *__restrict__ Y,
     long long ldx, long long ldy, float *__restrict__ out, const int *__restrict__ starts,
-    long long w, int blk) {
+    long long w, int blk, bool x_first) {
   constexpr int P = 32 / G;
   using Dv = Dense<XT, V>;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int g = lane / G, gl = lane & (G - 1);
   const uint64_t pol = l2_policy_evict_normal();
-  const uint64_t polx = sddmm_policy_x();
+  const uint64_t polx = sddmm_policy_x(x_first);
   const long long pb = w * blk;
   const long long pe = pb + blk < nnz ? pb + blk : nnz;
   int mcn = pb + lane < pe ? ld_stream(col + pb + lane) : 0;
@@ -401,11 +401,11 @@ __global__ void __launch_bounds__(kCta, 4) sddmm_fixed_kernel(
     int M, long long nnz, const int *__restrict__ row_ptr, const int *__restrict__ col,
     const float *__restrict__ val, const XT *__restrict__ X, const XT *__restrict__ Y,
     long long ldx, long long ldy, float *__restrict__ out, const int *__restrict__ starts,
-    long long nblk, int blk) {
+    long long nblk, int blk, bool x_first) {
   const long long w = (long long)blockIdx.x * (kCta / 32) + threadIdx.x / 32;
   if (w >= nblk) return;  // whole warp leaves together
   sddmm_fixed_block<XT, V, G, KI>(M, nnz, row_ptr, col, val, X, Y, ldx, ldy, out, starts, w,
-                                  blk);
+                                  blk, x_first);
 }
 
 // Several problems of one shape in one launch: warp w takes block
@@ -426,7 +426,8 @@ __global__ void __launch_bounds__(kCta, 4) sddmm_fixed_multi_kernel(
   const SddmmProblem &a = probs[lo];
   sddmm_fixed_block<XT, V, G, KI>(a.M, a.nnz, a.row_ptr, a.col, a.val,
                                   static_cast<const XT *>(a.X), static_cast<const XT *>(a.Y),
-                                  a.ldx, a.ldy, a.out, a.starts, w - a.blk_begin, kSddmmBlock);
+                                  a.ldx, a.ldy, a.out, a.starts, w - a.blk_begin, kSddmmBlock,
+                                  false);
 }
 
 // Blocks of at most P nonzeros per warp that fill whole waves of resident warps, so that
@@ -545,14 +546,14 @@ namespace {
 int launch_fixed_single(const SddmmShape &sh, int x_dtype, dim3 grid, int M, long long nnz,
                         const int *row_ptr, const int *col, const float *val, const void *X,
                         const void *Y, long long ldx, long long ldy, float *out, const int *starts,
-                        long long nblk, int blk, cudaStream_t s) {
+                        long long nblk, int blk, bool x_first, cudaStream_t s) {
 #define CASE_(XT, V, KI, G)                                                                \
   {                                                                                        \
     SddmmGrid b{blk, nblk, grid.x};                                                        \
     if (!starts) b = sddmm_grid<&sddmm_fixed_kernel<XT, V, G, KI>>(nnz, blk);              \
     sddmm_fixed_kernel<XT, V, G, KI><<<b.ctas, kCta, 0, s>>>(                              \
         M, nnz, row_ptr, col, val, static_cast<const XT *>(X), static_cast<const XT *>(Y), ldx, \
-        ldy, out, starts, b.nblk, (int)b.blk);                                             \
+        ldy, out, starts, b.nblk, (int)b.blk, x_first);                                    \
   }
   SEGTACO_SDDMM_SWITCH(sh, x_dtype)
 #undef CASE_
@@ -593,7 +594,7 @@ int launch_fixed_multi(const SddmmShape &sh, int x_dtype, dim3 grid, const Sddmm
     sddmm_gather_kernel<XT, E, C, G, F><<<b.ctas, kCta, 0, s>>>(                           \
         M, (unsigned)nnz, row_ptr, col, val, static_cast<const XT *>(X),                   \
         static_cast<const XT *>(Y), (unsigned)(ldx * sizeof(XT)), (unsigned)(ldy * sizeof(XT)), \
-        D, out, (unsigned)b.nblk, (unsigned)b.blk);                                        \
+        D, out, (unsigned)b.nblk, (unsigned)b.blk, x_first);                               \
   }
 #define SEGTACO_SDDMM_NARROW_CASE(XT, E, C, G)  \
   case SEGTACO_SDDMM_KEY(E, C, G):              \
@@ -607,6 +608,17 @@ int launch_fixed_multi(const SddmmShape &sh, int x_dtype, dim3 grid, const Sddmm
       SEGTACO_SDDMM_RUN(XT, E, C, G, false)     \
     break;
 
+// X and Y from 64 MB on do not stay in L2 beside the pattern, the results and what runs
+// between the calls.  Measured on GB300, repeated calls, X normal / leaving first: 90,000
+// lognormal rows, D = 128 bf16 (46 MB) 32.0 / 34.3 us; 100,000 power-law rows, D = 64 fp32
+// (51 MB) 45 / 49, 100 bf16 (40 MB) 73 / 82; 300,000, D = 64 bf16 (77 MB) 115.6 / 114.2, 32
+// fp32 (77 MB) 103.2 / 101.5, 128 bf16 (154 MB) 185 / 180; 90,000 lognormal rows, D = 128 fp32
+// (92 MB) 49.4 / 46.3, 400,000 (410 MB) 296 / 290.  (The choice in the kernel costs nothing.)
+bool sddmm_x_first(int M, int K, int D, int x_dtype) {
+  const long long esz = x_dtype == SEGTACO_BF16 ? 2 : 4;
+  return ((long long)M + K) * D * esz > (64LL << 20);
+}
+
 bool sddmm_gather_applies(int x_dtype, long long ldx, long long ldy) {
   const int esz = x_dtype == SEGTACO_BF16 ? 2 : 4;
   return ldx * esz < (1LL << 32) && ldy * esz < (1LL << 32);
@@ -615,7 +627,7 @@ bool sddmm_gather_applies(int x_dtype, long long ldx, long long ldy) {
 int launch_sddmm_gather(int M, long long nnz, const int *row_ptr, const int *col,
                         const float *val, const void *X, const void *Y, int x_dtype,
                         long long ldx, long long ldy, int D, float *out, int P,
-                        cudaStream_t s) {
+                        bool x_first, cudaStream_t s) {
   const int esz = x_dtype == SEGTACO_BF16 ? 2 : 4;
   const uintptr_t al = (uintptr_t)X | (uintptr_t)Y;
   int E = 32 / esz;
@@ -663,7 +675,7 @@ int launch_sddmm_gather(int M, long long nnz, const int *row_ptr, const int *col
 int launch_sddmm(int M, long long nnz, const int *row_ptr, const int *col, const float *val,
                  const void *X, const void *Y, int x_dtype, long long ldx, long long ldy, int D,
                  float *out, int *starts, int P, long long nblk, cudaStream_t s,
-                 bool starts_ready, int lanes, int kernel) {
+                 bool starts_ready, int lanes, int kernel, bool x_first) {
   if (nnz == 0) return SEGTACO_OK;
   if (!starts_ready && starts)
     SEGTACO_TRY(launch_block_starts_canonical(row_ptr, M, P, nblk, starts, s));
@@ -674,7 +686,7 @@ int launch_sddmm(int M, long long nnz, const int *row_ptr, const int *col, const
   const SddmmShape sh = sddmm_shape(x_dtype, D, ldx, ldy, X, Y, lanes);
   if (sh.family != 0 && kernel != SEGTACO_SDDMM_GENERAL)
     return launch_fixed_single(sh, x_dtype, grid, M, nnz, row_ptr, col, val, X, Y, ldx, ldy, out,
-                               starts, nblk, P, s);
+                               starts, nblk, P, x_first, s);
   const int V = sh.V;
   // Lanes per dot product: enough to cover D in one pass, at most 32.
   int G = 1;
