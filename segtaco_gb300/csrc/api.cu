@@ -1,5 +1,8 @@
 // api.cu -- the extern "C" entry points of include/segtaco.h, argument checks,
 // scratch handling and the SpMM planner (schedule / slab width / vector width).
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cstdarg>
@@ -42,36 +45,71 @@ int check_launch(const char *what) { return check_cuda(cudaGetLastError(), what)
 constexpr unsigned long long kScratchKeep = 64ull << 20;
 constexpr int kMaxDevices = 64;
 static std::mutex g_scratch_mu;
-static std::atomic<cudaMemPool_t> g_scratch_pool[kMaxDevices];
+// A device's pool and the id of the context that it was made in: cudaDeviceReset ends
+// both, and the next call makes another.
+struct ScratchPool {
+  std::atomic<unsigned long long> context{0};
+  std::atomic<cudaMemPool_t> pool{nullptr};
+};
+static ScratchPool g_scratch_pool[kMaxDevices];
+
+// Id of the current context; 0 where there is none.
+static unsigned long long context_id() {
+  static const auto get = [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+    return reinterpret_cast<PFN_cuCtxGetId_v12000>(p);
+  }();
+  unsigned long long id = 0;
+  return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
 
 // The current device's pool; nullptr where there is none (the caller then
 // allocates from the default pool).
 static cudaMemPool_t scratch_pool() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
-  cudaMemPool_t pool = g_scratch_pool[dev].load(std::memory_order_acquire);
-  if (pool) return pool;
+  const unsigned long long id = context_id();
+  if (id == 0) return nullptr;
+  ScratchPool &slot = g_scratch_pool[dev];
+  if (slot.context.load(std::memory_order_acquire) == id)
+    return slot.pool.load(std::memory_order_relaxed);
   std::lock_guard<std::mutex> lk(g_scratch_mu);
-  pool = g_scratch_pool[dev].load(std::memory_order_acquire);
-  if (pool) return pool;
+  if (slot.context.load(std::memory_order_acquire) == id)
+    return slot.pool.load(std::memory_order_relaxed);
   cudaMemPoolProps props{};
   props.allocType = cudaMemAllocationTypePinned;
   props.handleTypes = cudaMemHandleTypeNone;
   props.location.type = cudaMemLocationTypeDevice;
   props.location.id = dev;
   unsigned long long keep = kScratchKeep;
+  cudaMemPool_t pool = nullptr;
   if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
   cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-  g_scratch_pool[dev].store(pool, std::memory_order_release);
+  slot.pool.store(pool, std::memory_order_relaxed);
+  slot.context.store(id, std::memory_order_release);
   return pool;
 }
 
 void trim_scratch_pools() {
-  for (auto &p : g_scratch_pool)
-    if (cudaMemPool_t pool = p.load(std::memory_order_acquire)) cudaMemPoolTrimTo(pool, 0);
+  std::lock_guard<std::mutex> lk(g_scratch_mu);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  for (int d = 0; d < kMaxDevices; ++d) {
+    const cudaMemPool_t pool = g_scratch_pool[d].pool.load(std::memory_order_relaxed);
+    if (!pool || cudaSetDevice(d) != cudaSuccess) continue;
+    if (g_scratch_pool[d].context.load(std::memory_order_acquire) == context_id())
+      cudaMemPoolTrimTo(pool, 0);
+  }
+  cudaSetDevice(dev);
 }
 
 Scratch::~Scratch() {
