@@ -6,11 +6,12 @@
 // into P equal runs, one per slot: every slot has the same number of gathers
 // whatever the row lengths are, so no slot waits for another's longer row and
 // short rows need no batch of their own.  A slot walks its run in storage order, four
-// nonzeros a step with their gathers in flight together; a step's terms of a row are
-// summed by themselves and then added to the row's sum, so that a long row is rounded
-// once a step instead of once a term (error against FP64, one chain per row / here:
-// 77,777 lognormal rows, N = 37 9.3e-8 / 6.6e-8, N = 128 9.9e-8 / 6.8e-8; 250,000
-// power-law rows, N = 64 2.6e-7 / 1.6e-7, for 0 to 2 % of the time):
+// nonzeros a step with their gathers in flight together; terms of a row are summed by
+// themselves, four or two at a time, and then added to the row's sum, so that a long row is
+// rounded once for them instead of once a term (error against FP64, one chain per row /
+// here: 77,777 lognormal rows, N = 37 9.3e-8 / 7.2e-8, N = 128 9.8e-8 / 6.9e-8; 60,000
+// power-law rows, N = 64 2.3e-7 / 1.6e-7; 0 to 3 % of the time, rows of 16 1 to 5 %
+// faster):
 //   * a row that begins and ends in the run is stored as it ends;
 //   * the first row end of a run whose row began earlier keeps its partial sum in
 //     shared memory, and the row still open at the run's end leaves its sum there
@@ -43,11 +44,14 @@
 // columns per lane (1.10 ms against 1.18).
 #pragma once
 
+#include <type_traits>
+
 #include "spmm_kernels.cuh"
 
 namespace segtaco {
 
 constexpr int kSplitStep = 4;  // positions per slot and step: one 16-byte index load
+template <int N> using Int = std::integral_constant<int, N>;
 
 // Shared memory of one warp, in 4-byte words: the columns and values of the
 // chunk's nonzeros (whole steps from a multiple of 4, and one step more), its row
@@ -106,11 +110,6 @@ __device__ __forceinline__ ChunkEdges search_edges(const SpmmArgs<BT> &a, long l
 // JOIN (rb_pr, spmm_join.cu): chunk w's sums of rows cut by its edges are stored in
 // a.piece_part -- two rows of a.piece_ld floats, the row it starts in, then the row
 // open at its end -- instead of being added to C.
-// Steps in which some row ends sum their terms by themselves too, but for 8 bf16 elements
-// per lane: their registers cost warps or spill, and the gathers' round trips need the
-// warps (bf16, N = 128, 36 warps without / 32 with: 400,000 lognormal rows 158 / 187 us,
-// 200,000 80 / 97).  Error against FP64, one chain per row / all but those steps / all, bf16,
-// N = 64: lognormal rows 8.5e-8 / 7.9e-8 / 6.4e-8, power-law 1.8e-7 / 1.5e-7 / 1.4e-7.
 template <typename BT, int E, int C, int G, bool JOIN = false>
 __device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, const ChunkEdges ce,
                                                 int slab, int lane, int D,
@@ -118,7 +117,7 @@ __device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, const Chu
   constexpr int P = 32 / G;
   constexpr int V = E * C;
   constexpr int S = kSplitStep;
-  constexpr bool kStepSums = E <= 4;
+  static_assert(S == 4, "a step is summed as four terms or two pairs");
   using Dn = Dense<BT, E>;
   const unsigned FULL = 0xffffffffu;
   int *cs = sm;
@@ -245,71 +244,71 @@ __device__ __forceinline__ void spmm_split_unit(const SpmmArgs<BT> &a, const Chu
     }
     const float4 v4 = *reinterpret_cast<const float4 *>(vs + q);
     const float vv[S] = {v4.x, v4.y, v4.z, v4.w};
-    // The step's terms of the open row, or (kStepSums false) the row's sum itself.
-    float terms[kStepSums ? V : 1];
-    float *part = kStepSums ? terms : acc;
-    auto add = [&](int u, bool begin) {
+    // acc += the `count` terms from `first` on, summed by themselves
+    auto add = [&](auto first, auto count) {
+      constexpr int U = decltype(first)::value, K = decltype(count)::value;
 #pragma unroll
       for (int c = 0; c < C; ++c)
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-          const float x = Dn::get(b[u][c], e);
-          part[c * E + e] = kStepSums && begin ? vv[u] * x : fmaf(vv[u], x, part[c * E + e]);
+          if constexpr (K == 1) {
+            acc[c * E + e] = fmaf(vv[U], Dn::get(b[U][c], e), acc[c * E + e]);
+          } else {
+            float x = vv[U] * Dn::get(b[U][c], e);
+#pragma unroll
+            for (int k = 1; k < K; ++k) x = fmaf(vv[U + k], Dn::get(b[U + k][c], e), x);
+            acc[c * E + e] += x;
+          }
         }
-    };
-    auto close = [&]() {
-      if constexpr (kStepSums) {
-#pragma unroll
-        for (int v = 0; v < V; ++v) acc[v] += terms[v];
-      }
-    };
-    auto clear = [&]() {
-      if constexpr (kStepSums) {
-#pragma unroll
-        for (int v = 0; v < V; ++v) terms[v] = 0.0f;
-      }
     };
     const int p = ybase + q;
+    auto ends_at = [&](int pos) {  // closes the rows that end there
+      if (__any_sync(FULL, pos == rend)) {
+        if (pos == rend) next_row(pos);
+        __syncwarp();
+      }
+    };
     if (t == steps || (t == 0 && ragged0) || (t == steps - 1 && ragged1)) {
       // positions outside the chunk, or runs that have ended
-      clear();
-#pragma unroll
-      for (int u = 0; u < S; ++u) {
-        if (p + u >= lo && p + u < hi) {
-          if (p + u == rend) {
-            close();
-            next_row(p + u);
-            clear();
-          }
-          add(u, false);
+      auto one = [&](auto first) {
+        constexpr int U = decltype(first)::value;
+        if (p + U >= lo && p + U < hi) {
+          if (p + U == rend) next_row(p + U);
+          add(first, Int<1>());
         }
-      }
-    } else if (__all_sync(FULL, p + S <= rend)) {  // no row ends in the step
-#pragma unroll
-      for (int c = 0; c < C; ++c)
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-          float x = vv[0] * Dn::get(b[0][c], e);
-#pragma unroll
-          for (int u = 1; u < S; ++u) x = fmaf(vv[u], Dn::get(b[u][c], e), x);
-          acc[c * E + e] += x;
-        }
+      };
+      one(Int<0>()), one(Int<1>()), one(Int<2>()), one(Int<3>());
       continue;
-    } else {
-#pragma unroll
-      for (int u = 0; u < S; ++u) {
-        if (__any_sync(FULL, p + u == rend)) {
-          if (p + u == rend) {
-            if (u > 0) close();
-            next_row(p + u);
-            if (u > 0) clear();
-          }
-          __syncwarp();
-        }
-        add(u, u == 0);
-      }
     }
-    close();
+    if (E <= 4) ends_at(p);
+    if (__all_sync(FULL, p + S <= rend)) {  // no row ends in the step
+      add(Int<0>(), Int<4>());
+    } else if constexpr (E <= 4) {  // two by two, cut where a row ends between them
+      auto pair = [&](auto first, auto second) {
+        constexpr int U = decltype(first)::value;
+        if (U > 0) ends_at(p + U);
+        if (__any_sync(FULL, p + U + 1 == rend)) {
+          add(first, Int<1>());
+          if (p + U + 1 == rend) next_row(p + U + 1);
+          __syncwarp();
+          add(second, Int<1>());
+        } else {
+          add(first, Int<2>());
+        }
+      };
+      pair(Int<0>(), Int<1>());
+      pair(Int<2>(), Int<3>());
+    } else {
+      // 8 bf16 elements per lane: one by one.  Two by two 250,000 power-law rows, bf16, N =
+      // 64 85 / 89 us, N = 128 144 / 150, for the same error (1.5e-7); lognormal rows
+      // 7.9e-8 / 7.3e-8.  All terms of a row kept apart until the step's end: 6.4e-8, but 64
+      // registers, and 400,000 lognormal rows, N = 128 158 / 187 us.
+      auto one = [&](auto first) {
+        ends_at(p + decltype(first)::value);
+        add(first, Int<1>());
+      };
+      one(Int<0>()), one(Int<1>()), one(Int<2>()), one(Int<3>());
+    }
   }
   if (lo < hi && rend <= hi) flush();
 
