@@ -21,14 +21,16 @@
 // kernels, K columns of Poisson lengths; one warp per column / lists read across the
 // cluster, without the prefetch, after a memset / here: 1M columns of mean 2, 1000 entries
 // 3.2 / 5.3 / 3.3 us, 100,000 11.2 / 7.6 / 5.2; mean 20, 10,000 5.3 / 7.3 / 5.1,
-// 100,000 18.8 / 20.7 / 17.2, 250,000 36.9 / 41.3 / 37.1; 300,000 of mean 100, 10,000 10.1 /
-// 11.7 / 9.9, 100,000 57.9 / 76.9 / 61.8; 1M Zipf lengths up to 50,000, 100,000 entries 655 /
-// 31.7 / 23.8.
+// 100,000 18.8 / 20.7 / 17.2, 250,000 36.9 / 41.3 / 36.7; 300,000 of mean 100, 10,000 10.1 /
+// 11.7 / 10.2, 100,000 57.9 / 76.9 / 63.5; 1M Zipf lengths up to 50,000, 100,000 entries 655 /
+// 31.7 / 23.8; 1M power-law rows by columns (adds meet in hot rows), 100,000 22.7 / 27.5 /
+// 23.9.
 // Without clusters (a CTA's warps share its long columns) the short columns' calls are
 // 0.5 to 2 us faster, the Zipf ones with 10,000 and 100,000 entries 20 and 38 us.
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 #include "internal.h"
@@ -182,16 +184,17 @@ int launch_spmspv(int M, int K, long long nnz, const int *col_ptr, const int *ro
     return check_cuda(cudaMemsetAsync(y, 0, (size_t)M * sizeof(float), s), "memset y");
   // Entries per warp, E: few of them hide the chain of loads behind other warps, many
   // fill the flat ranges of short columns and save warps.  Up to 2048 entries one;
-  // beyond, E = sqrt(nx / 22 m) for columns of mean length m.  Measured on GB300, E = 3 / 6 /
-  // 11 / 15 / 24: 10,000 entries, m = 2 4.9 / 4.6 / 4.5 / 4.6 / 4.7 us, 20 5.3 / 5.8 / 6.0 /
-  // 6.8 / 8.0, 100 10.2 / 10.9 / 12.5 / 15.2 / 21; 100,000 entries, 2 17.9 / 11.0 / 8.0 / 5.9 /
-  // 5.5, 20 23.7 / 20.1 / 18.3 / 16.9 / 17.4, 100 62 / 62 / 63 / 66 / 68; 300,000 entries, 2 46 /
-  // 26 / 15.8 / 12.5 / 9.8, 20 63 / 49 / 43 / 41 / 40.  1000 entries, E = 1 / 3 / 8: 2 3.7 /
-  // 4.0 / 4.3, 100 4.3 / 6.3 / 9.5.
+  // beyond, E = sqrt(nx / 98 sqrt(m)) for columns of mean length m.  Measured on GB300, E = 3
+  // / 6 / 11 / 15 / 24: 10,000 entries, random rows, m = 2 4.9 / 4.6 / 4.5 / 4.6 / 4.7 us, 20
+  // 5.3 / 5.8 / 6.0 / 6.8 / 8.0, 100 10.2 / 10.9 / 12.5 / 15.2 / 21; 100,000 entries, 2 17.9 /
+  // 11.0 / 8.0 / 5.9 / 5.5, 20 23.7 / 20.1 / 18.3 / 16.9 / 17.4, 100 62 / 62 / 63 / 66 / 68,
+  // banded (72) 31.0 / 24.9 / 23.0 / 21.8 / 24; 300,000 entries, 2 46 / 26 / 15.8 / 12.5 / 9.8,
+  // 20 63 / 49 / 43 / 41 / 40.  1000 entries, E = 1 / 3 / 8: 2 3.7 / 4.0 / 4.3, 100 4.3 / 6.3 /
+  // 9.5.
   const double mean = K > 0 && nnz > K ? (double)nnz / K : 1.0;
   int per_warp = 1;
-  while (nx > 2048 && per_warp < 32 && 22.0 * mean * (per_warp + 1) * (per_warp + 1) <= nx)
-    ++per_warp;
+  const double unit = 98.0 * std::sqrt(mean);
+  while (nx > 2048 && per_warp < 32 && unit * (per_warp + 1) * (per_warp + 1) <= nx) ++per_warp;
   const long long vecs = (long long)M / 4, each = kCta * 4;
   const long long blocks = std::min<long long>(8LL * device_sms(), (vecs + each - 1) / each);
   clear_y_kernel<<<(unsigned)std::max<long long>(blocks, 1), kCta, 0, s>>>(y, (unsigned)M);
