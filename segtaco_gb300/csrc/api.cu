@@ -746,8 +746,8 @@ int segtaco_autotune_heuristic(int32_t M, int32_t K, int64_t nnz, int32_t N, int
   // rb_pr takes the band kernel (32-row blocks, the band of A as a dense tile,
   // B's window by TMA, 4 x 4 register tiles; spmm_window.cu) with a halo of
   // 32.  Measured on GB300, banded-plus-random 262,144 rows (half band 32, 8
-  // off-band nonzeros per row): fp32 N = 64 0.2465 -> 0.181 ms, bf16 B
-  // 0.2323 -> 0.114 ms, fp32 N = 128 0.650 -> 0.455 ms (halo 16: 0.61 ms,
+  // off-band nonzeros per row): fp32 N = 64 0.2465 -> 0.178 ms, bf16 B
+  // 0.2323 -> 0.112 ms, fp32 N = 128 0.650 -> 0.455 ms (halo 16: 0.61 ms,
   // 48: 0.29 ms at fp32 N = 64).  The staged window for the row-block walk
   // (still one gathered B slice per nonzero, from shared memory instead of
   // L1) measured slower than the plain row blocks (0.373 vs 0.248 ms) and is
@@ -983,7 +983,7 @@ int segtaco_sddmm_autotune(int32_t M, int32_t K, int64_t nnz, int32_t D, int32_t
   cfg->kernel = SEGTACO_SDDMM_AUTO;
   // Rows known to lie near the diagonal: the band kernel (sddmm_band.cu).
   // Measured on GB300, banded-plus-random 262,144 rows, D = 64: fp32 0.330 ->
-  // 0.194 ms, bf16 factors 0.303 -> 0.150 ms.
+  // 0.191 ms, bf16 factors 0.303 -> 0.150 ms.
   if (banded && D == 64) cfg->kernel = SEGTACO_SDDMM_BAND;
   (void)x_dtype;
   // Blocks of 256 nonzeros per warp; smaller for small problems, so that the

@@ -1,5 +1,5 @@
 // mma.cuh -- warp-level tensor-core steps of the band kernels (bf16 operands, fp32
-// accumulation) and the exact split of fp32 values into bf16 parts.
+// accumulation) and the split of fp32 values into bf16 parts.
 #pragma once
 
 #include <stdint.h>

@@ -28,8 +28,8 @@
 // What bounds it: the sampling of the tile and the off-band gathers, each about half
 // of what the product leaves (without the off-band list 136 us, without the product
 // 158).  Measured on GB300, banded-plus-random 262,144 rows, half band 32, 8 off-band
-// nonzeros per row, multiply-adds on 4 x 6 register tiles -> here: fp32 246 -> 194 us,
-// bf16 222 -> 150; error against FP64 1.4e-7 -> 9.7e-8 and 5.0e-8 -> 4.6e-8.  Eight
+// nonzeros per row, multiply-adds on 4 x 6 register tiles -> here: fp32 246 -> 191 us,
+// bf16 222 -> 150; error against FP64 1.4e-7 -> 6.0e-8 and 5.0e-8 -> 4.6e-8.  Eight
 // off-band steps in flight instead of four 206 -> 195 us; 20 sampled nonzeros in flight
 // instead of 10 spill (258); a warp per row in the sampling 252.
 #include <cfloat>

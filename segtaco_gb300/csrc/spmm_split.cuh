@@ -30,7 +30,7 @@
 // N) up to four 1- or 2-element chunks per lane on 8, 16 or 32 lanes, so that one
 // pass over A covers up to 128 columns.
 //
-// What bounds it: the gathers' round trips to L2 (30 warps per SM, 56 % of issue
+// What bounds it: the gathers' round trips to L2 (31 warps per SM, 60 % of issue
 // slots used, long-scoreboard stalls first; 12.9 TB/s of gathers on 250,000
 // power-law rows, N = 64, against ~17 TB/s for bare random 128-byte rows).  Eight
 // loads in flight per lane cost registers and L1 and were slower (115 us against

@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kSpmmCta, 5)
 // The tile product At x B is a dense contraction (32 x win by win x 64 per CTA), and
 // its multiply-adds, two shared loads per 16 of them, were the kernel's time.  Here
 // it runs as mma.m16n8k16 with fp32 accumulation.  A's values are fp32: each is split
-// exactly into three bf16 parts (x = hi + mid + lo, mma.cuh), so three
+// into three bf16 parts (x = hi + mid + lo, mma.cuh), so three
 // products per step give the exact products x*b that the multiply-add form rounds
 // once; the parts of a step are summed from zero, lowest first, and added to the
 // running sum in fp32.  (tcgen05 needs 64 or 128 rows per tile: a 32-row block's
@@ -364,10 +364,10 @@ __global__ void __launch_bounds__(kSpmmCta, 5)
 // parts: a CTA that finds an infinity or NaN among its sums, or such a value in its
 // tile, sums its rows nonzero by nonzero instead.
 //
-// What bounds it now: instructions (58 % of issue slots with 24 warps per SM), most of
+// What bounds it now: instructions (56 % of issue slots with 23 warps per SM), most of
 // them in the scatter and the off-band rows; the tensor pipe is 14 % busy.  Measured
 // on GB300, banded-plus-random 262,144 rows (half band 32, 8 off-band nonzeros per
-// row), bf16 B, N = 64: 160 us with multiply-adds -> 114 (without the product 97,
+// row), bf16 B, N = 64: 160 us with multiply-adds -> 112 (without the product 97,
 // without the off-band rows 97); error against FP64 1.5e-7 -> 9.3e-8.  20 nonzeros in
 // flight per thread instead of 10 117.5 -> 115.6 us; a warp per row instead of the flat
 // scatter 122; seven CTAs per SM 120; all three parts summed in the tensor cores'
